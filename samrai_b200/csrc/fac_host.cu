@@ -322,6 +322,7 @@ struct LevelState {
    DevArray<long long> facemap;
    DevArray<int> pushmap;
    std::vector<int> pushmap_h;  // host copy (face masks of the staged units)
+   std::vector<long long> facemap_h;  // host copy, level 0 while its solve is built
    // side-array faces that carry a coarsened finer-level flux
    DevArray<unsigned char> fcmask;
    bool fused_ok = false;
@@ -381,10 +382,11 @@ struct LevelState {
    DevArray<double> tmp;
    DevArray<double> dxc_prob;                        // per problem dx of level ln-1
    DevArray<unsigned long long> maxres_red, maxres_blk;
-   bool one_patch_per_prob = false;  // patch p is problem p's only patch, <= 16384 cells
-   bool facemap_local = false;       // no face of the level has a same-level neighbour
-   int solve_smem = 0;               // shared bytes of the one-launch solve on shared
-                                     // copies (0: that form does not fit)
+   // level 0: the one-launch coarsest solve (build_coarse_solve); ncta = 0:
+   // the level does not fit it
+   int coarse_ncta = 0, coarse_sp = 0, coarse_smem = 0;
+   DevArray<unsigned char> d_coarse;  // its tables, one after another
+   size_t coarse_at[5] = {0, 0, 0, 0, 0};  // halo, CTAs, cells, pushes, ghosts
    DevArray<int> last_patch;
    std::vector<long long> dir_idx;
    DevArray<long long> d_dir_idx;
@@ -1419,13 +1421,295 @@ void build_facemap(fac_ctx *c, int ln)
          throw FacError(FAC_ERR_NESTING, "face table disagrees with the coarse-fine boundary");
    }
    L.fused_ok = ok;
-   L.facemap_local = true;
-   for (long long t = 0; t < L.no; ++t)
-      if (fmap[t] >= 0) L.facemap_local = false;
    L.facemap.upload(fmap, c->stream);
+   if (ln == 0) L.facemap_h = std::move(fmap);
    L.pushmap.upload(pmap, c->stream);
    L.pushmap_h = std::move(pmap);
    build_stage_units(c, ln);
+}
+
+// Tables of the one-launch coarsest solve (fac_coarse.cu) for ncta CTAs per
+// problem: each problem's level-0 cells, in patch and storage order, in ncta
+// equal runs.  False when a CTA would hold more than sp cells of one colour
+// per thread, or its shared values do not fit.
+struct CoarseTables {
+   std::vector<CoarseCta> ctas;
+   std::vector<CoarseCell> cells;
+   std::vector<long long> halo;
+   std::vector<unsigned> push, ghost;
+   int smem = 0;
+};
+
+bool build_coarse_tables(const fac_ctx *c, int ncta, int sp, CoarseTables &T)
+{
+   const LevelState &L = c->L[0];
+   const int dim = c->dim;
+   T = CoarseTables();
+   for (int p = 0; p < nprob(c); ++p) {
+      const int pb = L.prob_patch_begin[p], pe = L.prob_patch_begin[p + 1];
+      const long long base = L.prob_off1[p];
+      long long N = 0;
+      for (int ip = pb; ip < pe; ++ip) N += L.box[ip].size();
+      // ordinal of every cell of the problem's slice of the ghost-1 field
+      std::vector<int> ord((size_t)(L.prob_off1[p + 1] - base), -1);
+      std::vector<int> owner((size_t)N), local((size_t)N);
+      std::vector<long long> where((size_t)N);  // ghost-1 element of each cell
+      std::vector<unsigned char> colour((size_t)N);
+      std::vector<int> ncol((size_t)ncta * 2, 0);
+      int q = 0;
+      for (int ip = pb; ip < pe; ++ip) {
+         const Box &b = L.box[ip];
+         const Box g = ghost_box(dim, b, 1);
+         const long long gx = g.hi[0] - g.lo[0] + 1, gy = g.hi[1] - g.lo[1] + 1;
+         for (int a = 0; a < dim; ++a)
+            if (b.lo[a] < 0) return false;  // the colour rule below is that of k_rbgs for these
+         for (int k = b.lo[2]; k <= b.hi[2]; ++k)
+            for (int j = b.lo[1]; j <= b.hi[1]; ++j)
+               for (int i = b.lo[0]; i <= b.hi[0]; ++i, ++q) {
+                  where[q] = L.hp[ip].off1 + (i - g.lo[0]) + gx * ((j - g.lo[1]) + gy * (k - g.lo[2]));
+                  ord[(size_t)(where[q] - base)] = q;
+                  owner[q] = (int)((long long)q * ncta / N);
+                  colour[q] = (unsigned char)((dim == 3 ? i + j + k : i - b.lo[0] + b.lo[1] + j) & 1);
+                  local[q] = ncol[2 * owner[q] + colour[q]]++;
+               }
+      }
+      for (int v : ncol)
+         if (v > kCoarseThreads * sp) return false;
+      // black cells after the red ones
+      for (int i = 0; i < (int)N; ++i)
+         if (colour[i]) local[i] += ncol[2 * owner[i]];
+      const int cta0 = (int)T.ctas.size();
+      std::vector<std::vector<CoarseCell>> mine(ncta);
+      std::vector<std::vector<long long>> halo(ncta);
+      // ghost values per CTA and colour: face << 16 | the cell's shared value
+      std::vector<std::vector<unsigned>> ghost(2 * ncta);
+      // CTAs a cell's value is pushed to: (rank, shared value there)
+      std::vector<std::vector<unsigned>> to((size_t)N);
+      std::vector<int> seen((size_t)N, -1), slot((size_t)N, 0);
+      for (int r = 0; r < ncta; ++r) {
+         mine[r].resize((size_t)ncol[2 * r] + ncol[2 * r + 1]);
+         CoarseCta ct = {};
+         ct.prob = p;
+         ct.rank = r;
+         ct.ncol[0] = ncol[2 * r];
+         ct.ncol[1] = ncol[2 * r + 1];
+         ct.patch0 = pb;
+         T.ctas.push_back(ct);
+      }
+      // first the copies a CTA needs and the ghost values of its red and black
+      // cells, then (their numbers known) where each ghost value is
+      std::vector<int> gnext(2 * ncta, 0);
+      for (int pass = 0; pass < 2; ++pass) {
+         q = 0;
+         for (int ip = pb; ip < pe; ++ip) {
+            const PatchDesc &d = L.hp[ip];
+            const Box &b = L.box[ip];
+            const int n[3] = {b.hi[0] - b.lo[0] + 1, b.hi[1] - b.lo[1] + 1, b.hi[2] - b.lo[2] + 1};
+            const long long step[3] = {1, n[0] + 2, (long long)(n[0] + 2) * (n[1] + 2)};
+            for (int lin = 0; lin < n[0] * n[1] * n[2]; ++lin, ++q) {
+               const int x[3] = {lin % n[0], lin / n[0] % n[1], lin / (n[0] * n[1])};
+               const int r = owner[q];
+               const int nown = ncol[2 * r] + ncol[2 * r + 1];
+               CoarseCell &ce = mine[r][local[q]];
+               ce.patch = ip;
+               ce.lin = lin;
+               if (ip == pe - 1) ce.last = (unsigned short)(T.ctas[cta0 + r].last = 1);
+               for (int fc = 0; fc < 2 * dim; ++fc) {
+                  const int a = fc >> 1, s = fc & 1;
+                  const long long next = where[q] + (s ? step[a] : -step[a]);
+                  long long m = next;
+                  if (x[a] == (s ? n[a] - 1 : 0)) {
+                     const int t = a == 0 ? x[1] + n[1] * x[2]
+                                          : (a == 1 ? x[0] + n[0] * x[2] : x[0] + n[0] * x[1]);
+                     m = L.facemap_h[d.offo[a][s] + t];
+                  }
+                  int at = -1;
+                  if (m >= 0) {
+                     const int w = ord[(size_t)(m - base)];
+                     if (w < 0) return false;
+                     if (owner[w] == r) {
+                        at = local[w];
+                     } else {
+                        if (pass == 0 && seen[w] != r) {
+                           // cells are visited CTA by CTA (owners ascend), so
+                           // seen and slot hold this CTA's copy
+                           seen[w] = r;
+                           slot[w] = nown + (int)halo[r].size();
+                           halo[r].push_back(m);
+                           T.ctas[cta0 + r].nin[colour[w]] += 1;
+                           to[w].push_back((unsigned)r << 16 | (unsigned)slot[w]);
+                        }
+                        at = pass == 0 ? slot[w] : (int)ce.nb[fc];
+                     }
+                  } else if (m == -2) {
+                     // not a cell of this level: the ghost value as it is
+                     if (pass == 0) {
+                        at = nown + (int)halo[r].size();
+                        halo[r].push_back(next);
+                     } else {
+                        at = ce.nb[fc];
+                     }
+                  } else if (pass == 0) {
+                     ghost[2 * r + colour[q]].push_back((unsigned)fc << 16 | (unsigned)local[q]);
+                     at = 0;
+                  } else {
+                     at = nown + (int)halo[r].size() + gnext[2 * r + colour[q]]++ +
+                          (colour[q] ? (int)ghost[2 * r].size() : 0);
+                  }
+                  if (at < 0 || at > 0xffff) return false;
+                  ce.nb[fc] = (unsigned short)at;
+               }
+            }
+         }
+      }
+      for (int i = 0; i < (int)N; ++i) {
+         CoarseCell &ce = mine[owner[i]][local[i]];
+         ce.npush = (unsigned short)to[i].size();
+      }
+      std::vector<std::vector<int>> cell_of(ncta);
+      for (int r = 0; r < ncta; ++r) cell_of[r].resize(mine[r].size());
+      for (int i = 0; i < (int)N; ++i) cell_of[owner[i]][local[i]] = i;
+      for (int r = 0; r < ncta; ++r) {
+         CoarseCta &ct = T.ctas[cta0 + r];
+         ct.cell0 = (int)T.cells.size();
+         ct.halo0 = (int)T.halo.size();
+         ct.push0 = (int)T.push.size();
+         ct.nhalo = (int)halo[r].size();
+         ct.ghost0 = (int)T.ghost.size();
+         for (int k = 0; k < 2; ++k) {
+            ct.nghost[k] = (int)ghost[2 * r + k].size();
+            T.ghost.insert(T.ghost.end(), ghost[2 * r + k].begin(), ghost[2 * r + k].end());
+         }
+         for (size_t k = 0; k < mine[r].size(); ++k) {
+            mine[r][k].push0 = (int)T.push.size() - ct.push0;
+            const auto &t = to[cell_of[r][k]];
+            T.push.insert(T.push.end(), t.begin(), t.end());
+         }
+         ct.npush = (int)T.push.size() - ct.push0;
+         T.cells.insert(T.cells.end(), mine[r].begin(), mine[r].end());
+         T.halo.insert(T.halo.end(), halo[r].begin(), halo[r].end());
+         const int ng = ct.nghost[0] + ct.nghost[1];
+         const long long nloc = (long long)mine[r].size() + ct.nhalo + ng;
+         const long long bytes = 8 * nloc + 8LL * ct.npush + 4LL * ng;
+         if (nloc > 0xffff || bytes > kSolveSmemMax) return false;
+         T.smem = std::max(T.smem, (int)((bytes + 15) / 16 * 16));
+      }
+   }
+   // every index the kernel forms stays inside its CTA's shared values, every
+   // push lands on a copy of its target CTA, every initial value in the field,
+   // and a CTA expects as many copies of a colour as are sent to it (its wait
+   // ends)
+   std::vector<int> sent(2 * T.ctas.size(), 0);
+   for (size_t b = 0; b < T.ctas.size(); ++b) {
+      const CoarseCta &ct = T.ctas[b];
+      for (int k = 0; k < ct.ncol[0] + ct.ncol[1]; ++k) {
+         const CoarseCell &ce = T.cells[(size_t)ct.cell0 + k];
+         for (int e = 0; e < ce.npush; ++e)
+            sent[2 * (b - ct.rank + (T.push[(size_t)ct.push0 + ce.push0 + e] >> 16)) +
+                 (k < ct.ncol[0] ? 0 : 1)] += 1;
+      }
+   }
+   for (size_t b = 0; b < T.ctas.size(); ++b)
+      for (int k = 0; k < 2; ++k)
+         if (sent[2 * b + k] != T.ctas[b].nin[k])
+            throw FacError(FAC_ERR_ARG, "coarsest-solve copies do not match what is sent");
+   for (size_t b = 0; b < T.ctas.size(); ++b) {
+      const CoarseCta &ct = T.ctas[b];
+      const int nown = ct.ncol[0] + ct.ncol[1];
+      const int nloc = nown + ct.nhalo + ct.nghost[0] + ct.nghost[1];
+      for (int k = 0; k < nown; ++k) {
+         const CoarseCell &ce = T.cells[(size_t)ct.cell0 + k];
+         bool ok = ce.push0 >= 0 && ce.push0 + ce.npush <= ct.npush && ce.npush < 128 &&
+                   ce.push0 < (1 << 24);
+         for (int fc = 0; fc < 2 * dim; ++fc) ok = ok && ce.nb[fc] < nloc;
+         if (!ok) throw FacError(FAC_ERR_ARG, "coarsest-solve cell out of range");
+      }
+      for (int k = 0; k < ct.npush; ++k) {
+         const unsigned t = T.push[(size_t)ct.push0 + k];
+         const int r = (int)(t >> 16), at = (int)(t & 0xffffu);
+         if (r >= ncta) throw FacError(FAC_ERR_ARG, "coarsest-solve push out of range");
+         const CoarseCta &to = T.ctas[b - ct.rank + r];
+         const int lo = to.ncol[0] + to.ncol[1];
+         if (at < lo || at >= lo + to.nhalo)
+            throw FacError(FAC_ERR_ARG, "coarsest-solve push out of range");
+      }
+      for (int k = 0; k < ct.nghost[0] + ct.nghost[1]; ++k)
+         if ((int)(T.ghost[(size_t)ct.ghost0 + k] & 0xffffu) >= nown)
+            throw FacError(FAC_ERR_ARG, "coarsest-solve ghost value out of range");
+      for (int k = 0; k < ct.nhalo; ++k) {
+         const long long m = T.halo[(size_t)ct.halo0 + k];
+         if (m < 0 || m >= L.n1) throw FacError(FAC_ERR_ARG, "coarsest-solve copy out of range");
+      }
+   }
+   return true;
+}
+
+// Time of a pass of the coarsest solve on ncta CTAs with up to sp cells of a
+// colour per thread, load on average: a fit to measurements (8^3..16^3, 30 x
+// 40..97 x 97, one problem): 0.3 us for the chain of a pass alone, 0.3 us more
+// once values cross CTAs, and per cell of a thread the FP64 and shared-memory
+// work, which grows where sp cells' coefficients no longer fit the registers.
+// Measured at 64^2: 1 CTA 0.90 us, 2 0.86, 4 0.74, 8 0.65, 16 0.70; at 16^3: 1
+// 2.14, 2 1.25, 4 0.81, 8 0.74, 16 0.80; for 64 problems of 16^3 at once 2 CTAs
+// each (one wave) 1.26, 4 (two waves) 1.63.
+double coarse_pass_us(int dim, int ncta, int sp, double load)
+{
+   const double base = ncta == 1 ? 0.3 : (ncta <= 4 ? 0.6 : (ncta == 8 ? 0.63 : 0.7));
+   const double cell = dim == 2 ? (sp == 1 ? 0.12 : (sp == 2 ? 0.15 : 0.18))
+                                : (sp == 1 ? 0.2 : (sp == 2 ? 0.3 : 0.45));
+   return base + cell * load;
+}
+
+void build_coarse_solve(fac_ctx *c)
+{
+   LevelState &L = c->L[0];
+   L.coarse_ncta = 0;
+   long long most = 0;
+   for (int p = 0; p < nprob(c); ++p) {
+      long long n = 0;
+      for (int ip = L.prob_patch_begin[p]; ip < L.prob_patch_begin[p + 1]; ++ip) n += L.box[ip].size();
+      if (n == 0) return;
+      most = std::max(most, n);
+   }
+   if (!L.fused_ok || most > 2LL * kCoarseThreads * kCoarseSlotsMax * kCoarseClusterMax) return;
+   struct Choice {
+      double cost;
+      int ncta, sp;
+   };
+   std::vector<Choice> choices;
+   for (int n = 1; n <= kCoarseClusterMax; n *= 2)
+      for (int sp = 1; sp <= kCoarseSlotsMax; sp *= 2) {
+         if (most > 2LL * kCoarseThreads * sp * n) continue;
+         const int at_once = g_dry ? 144 / n : coarse_solve_clusters(c->dim, c->spec, n, sp);
+         if (at_once <= 0) continue;
+         const int waves = (nprob(c) + at_once - 1) / at_once;
+         choices.push_back(
+            {waves * coarse_pass_us(c->dim, n, sp, 0.5 * (double)most / n / kCoarseThreads), n, sp});
+      }
+   std::stable_sort(choices.begin(), choices.end(),
+                    [](const Choice &x, const Choice &y) { return x.cost < y.cost; });
+   CoarseTables T;
+   for (const Choice &ch : choices) {
+      if (!build_coarse_tables(c, ch.ncta, ch.sp, T)) continue;
+      L.coarse_ncta = ch.ncta;
+      L.coarse_sp = ch.sp;
+      L.coarse_smem = T.smem;
+      std::vector<unsigned char> all;
+      auto append = [&](int k, const void *src, size_t bytes) {
+         L.coarse_at[k] = all.size();
+         all.resize((all.size() + bytes + 15) / 16 * 16);
+         if (bytes) memcpy(all.data() + L.coarse_at[k], src, bytes);
+      };
+      append(0, T.halo.data(), T.halo.size() * sizeof(long long));
+      append(1, T.ctas.data(), T.ctas.size() * sizeof(CoarseCta));
+      append(2, T.cells.data(), T.cells.size() * sizeof(CoarseCell));
+      append(3, T.push.data(), T.push.size() * sizeof(unsigned));
+      append(4, T.ghost.data(), T.ghost.size() * sizeof(unsigned));
+      L.d_coarse.upload(all, c->stream);
+      break;
+   }
+   L.facemap_h.clear();
+   L.facemap_h.shrink_to_fit();
 }
 
 void build_chunks(fac_ctx *c, int ln)
@@ -1495,24 +1779,6 @@ void build_chunks(fac_ctx *c, int ln)
    L.last_patch.upload(last, c->stream);
    L.maxres_red.alloc(std::max(1, L.npatch));
    L.maxres_blk.alloc(std::max(1, L.npatch));
-   // one block per problem pays off for small patches only
-   L.one_patch_per_prob = L.npatch == np;
-   for (int ip = 0; ip < L.npatch; ++ip)
-      if (L.hp[ip].prob != ip || L.box[ip].size() > 16384) L.one_patch_per_prob = false;
-   // the one-launch solve on shared copies of u, f, D and C (FP64)
-   L.solve_smem = 0;
-   if (L.one_patch_per_prob && L.facemap_local) {
-      long long most = 0;
-      for (int ip = 0; ip < L.npatch; ++ip) {
-         const Box &b = L.box[ip];
-         long long n = cell_count(c->dim, b, 1) + b.size();
-         if (c->spec.d_variable)
-            for (int a = 0; a < c->dim; ++a) n += side_box(b, a).size();
-         if (c->spec.c_kind == 2) n += b.size();
-         most = std::max(most, 8 * n);
-      }
-      if (most <= kSolveSmemMax) L.solve_smem = (int)most;
-   }
    // one colour pass reads u over the ghosted boxes, f at the active half,
    // writes u at the active half, and reads D on all faces when variable
    double n = 0, ng = 0;
@@ -2194,6 +2460,7 @@ void initialize(fac_ctx *c)
       build_res_units(c, ln);
       build_residual_fixups(c, ln);
    }
+   build_coarse_solve(c);
    validate_tables(c);
    for (int ln = 0; ln < c->nlev; ++ln) {
       LevelState &L = c->L[ln];
@@ -2265,15 +2532,19 @@ void smooth(fac_ctx *c, int fid_e, int fid_r, int ln, int nsweeps, double tol)
    if (ln > 0) ghost_fill(c, fid_e, ln, true, 1, c->run.p);
    else if (!fmap || staged) ghost_fill(c, fid_e, ln, false, 1, c->run.p);
    std::vector<int> hrun(np);
-   // smoothing to a tolerance on a level without a coarser one and with one
-   // patch per problem (the coarsest level): every sweep in one launch
-   const bool one_launch = tol >= 0.0 && ln == 0 && fmap && L.one_patch_per_prob;
+   // smoothing to a tolerance on the coarsest level: every sweep in one launch
+   const bool one_launch = tol >= 0.0 && ln == 0 && fmap && L.coarse_ncta > 0;
    if (one_launch) {
       const int pi = prof_begin(c, 0, L.rb_bytes_prob, 2.0 * nsweeps);
-      launch_rbgs_solve<double>(c->stream, c->dim, c->spec, L.npatch, L.d_patches.p, e, r,
-                                L.d.p, L.c.p, fmap, c->bc, nsweeps, tol, c->run.p,
-                                c->sweeps_call.p, L.maxres_red.p, L.maxres_blk.p,
-                                L.solve_smem);
+      const unsigned char *t = L.d_coarse.p;
+      CUDA_CHECK(launch_coarse_solve(
+         c->stream, c->dim, c->spec, np, L.coarse_ncta, L.coarse_sp, L.coarse_smem,
+         reinterpret_cast<const CoarseCta *>(t + L.coarse_at[1]),
+         reinterpret_cast<const CoarseCell *>(t + L.coarse_at[2]),
+         reinterpret_cast<const long long *>(t + L.coarse_at[0]),
+         reinterpret_cast<const unsigned *>(t + L.coarse_at[3]),
+         reinterpret_cast<const unsigned *>(t + L.coarse_at[4]), L.d_patches.p, e, r, L.d.p, L.c.p,
+         c->bc, nsweeps, tol, c->run.p, c->sweeps_call.p, c->kerr.p));
       prof_end(c, pi);
    }
    for (int isweep = 0; isweep < (one_launch ? 0 : nsweeps); ++isweep) {
@@ -4320,10 +4591,6 @@ int fac_ctx_create(fac_ctx **ctx, int dim, int device)
          CUDA_CHECK(cudaGetDeviceCount(&ndev));
          if (device >= ndev) throw FacError(FAC_ERR_ARG, "bad device index");
          CUDA_CHECK(cudaSetDevice(device));
-         // outside any stream capture: the shared-memory limit of the
-         // one-launch coarsest solve (stays set for the process)
-         if (!allow_solve_smem(kSolveSmemMax))
-            throw FacError(FAC_ERR_CUDA, "shared-memory limit of the coarsest solve refused");
       }
       fac_ctx *c = new fac_ctx();
       c->dim = dim;

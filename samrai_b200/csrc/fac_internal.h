@@ -163,8 +163,8 @@ struct WaitTest {
 
 // Largest dynamic shared memory of one CTA of the staged colour pass.
 constexpr int kStageSmemMax = 227 * 1024;
-// dynamic shared memory of the one-launch coarsest solve on shared copies
-// (its static reduction array takes part of the per-block limit)
+// dynamic shared memory of a CTA of the coarsest solve (its static part takes
+// some of the per-block limit)
 constexpr int kSolveSmemMax = kStageSmemMax - 1024;
 // staged pass: mbarriers and copy sources ahead of the stages, and the
 // largest ring of stages a CTA holds
@@ -410,6 +410,36 @@ struct UnitCopy {
    int nbytes;
    int dst_off;
    int total;
+};
+
+// Coarsest-level solve by one thread-block cluster per problem
+// (fac_coarse.cu): threads of a CTA and the cells of each colour a thread
+// may own (compiled for 1, 2 and 4).
+constexpr int kCoarseThreads = 512;
+constexpr int kCoarseSlotsMax = 4;
+constexpr int kCoarseClusterMax = 16;
+
+// One CTA: its own cells are cells[cell0 ..], the ncol[0] red ones first,
+// and its shared values are those cells, nhalo copies of cells other CTAs
+// own (or fixed ghost values), then the physical-boundary ghost values of its
+// red and of its black cells.
+struct CoarseCta {
+   int prob, patch0, rank;
+   int cell0, ncol[2];
+   int nhalo, halo0;    // initial values: elements halo[halo0 ..] of the ghost-1 field
+   int nin[2];          // copies of each colour that other CTAs keep current
+   int nghost[2], ghost0;  // ghost[ghost0 ..]: face << 16 | shared value of the cell
+   int npush, push0;    // push targets: CTA rank << 16 | index of its shared value
+   int last;            // holds cells of the problem's last patch
+};
+
+struct CoarseCell {
+   int patch;
+   int lin;                // cell of the patch, x fastest
+   unsigned short nb[6];   // shared values behind the low and high face of each axis
+   unsigned short npush;
+   unsigned short last;    // 1: a cell of the problem's last patch
+   int push0;              // first push entry, from the CTA's push0
 };
 
 struct PoissonSpec {

@@ -116,23 +116,20 @@ template <class T>
 void launch_fill(cudaStream_t s, const FillItem *items, const Chunk *chunks, int nchunks,
                  const int *prefix, T *dst, const T *src_same, const T *src_coarse, int homogeneous,
                  const BcCoefs &bc, const int *active);
-// Red-black smoothing to a tolerance, all sweeps in one launch, of a level
-// without a coarser level and with one patch per problem (patch b of
-// problem patches[b].prob); run, sweeps and the per-patch red / black
-// residual maxima as the per-pass launches and the sweep check leave them.
-// smem > 0: every patch's arrays fit that many bytes of shared memory and
-// the face table has no same-level neighbour; the sweeps run on shared
-// copies (same bits).
-// Let the shared-memory form of the one-launch solve (FP64) take up to
-// `bytes` of dynamic shared memory on the current device; false if refused.
-bool allow_solve_smem(int bytes);
-template <class T>
-void launch_rbgs_solve(cudaStream_t s, int dim, const PoissonSpec &spec, int npatch,
-                       const PatchDesc *patches, T *u, const T *f, const T *dside,
-                       const T *cfield, const long long *facemap, const BcCoefs &bc,
-                       int nsweeps, double tol, int *run, long long *sweeps,
-                       unsigned long long *maxres_red, unsigned long long *maxres_blk,
-                       int smem = 0);
+// Red-black smoothing to a tolerance of a level without a coarser level, all
+// sweeps in one launch: ncta CTAs per problem form a cluster, sp cells of each
+// colour per thread, smem bytes of shared memory per CTA (fac_coarse.cu); run
+// and sweeps as the per-pass launches and the sweep check leave them.
+// coarse_solve_clusters: how many such clusters the current device runs at
+// once, 0 for none (sets the kernel's limits; call it outside stream capture).
+int coarse_solve_clusters(int dim, const PoissonSpec &spec, int ncta, int sp);
+cudaError_t launch_coarse_solve(cudaStream_t s, int dim, const PoissonSpec &spec, int nprob,
+                                int ncta, int sp, int smem, const CoarseCta *ctas,
+                                const CoarseCell *cells, const long long *halo,
+                                const unsigned *push, const unsigned *ghost,
+                                const PatchDesc *patches, double *u, const double *f,
+                                const double *dside, const double *cfield, const BcCoefs &bc,
+                                int nsweeps, double tol, int *run, long long *sweeps, int *err);
 // Ghost fill from a gather list of n elements (copies and constant refines,
 // see k_fill_gather) plus the physical-boundary items of the same fill.
 template <class T>
