@@ -78,3 +78,62 @@ def test_batch_walk_matches_single_samples(require_gpu):
         assert torch.equal(ys, y[first:first + 2])
     assert torch.isfinite(y).all()
     net.close()
+
+
+@pytest.mark.parametrize("n", [1, 3])
+def test_fractional_masks_match_oracle(n, require_gpu):
+    """Masks that are no 0/1 fields (their sum is formed on the device), on
+    data of two scales; the bounds of the test above."""
+    import torch
+    rng = np.random.default_rng(10 + n)
+    ref = co.CNN.init(seed=4)
+    x = rng.standard_normal((n, S, S, S)).astype(np.float32)
+    t = (1e-3 * rng.standard_normal((n, S, S, S))).astype(np.float32)
+    mask = rng.random((n, S, S, S)).astype(np.float32)
+    net = fac.CNN(max_batch=n)
+    net.set_weights(ref.w)
+    xd, td, md = (torch.from_numpy(a).cuda() for a in (x, t, mask))
+    loss, gs = net.gradients(xd.data_ptr(), td.data_ptr(), md.data_ptr(), n)
+    loss_ref, gs_ref = ref.loss_and_grads(x, t, mask)
+    assert abs(loss - loss_ref) <= 1e-2 * loss_ref
+    for g, gr in zip(gs, gs_ref):
+        assert rel(g, gr) < 3e-2, rel(g, gr)
+    with pytest.raises(fac.FacError):
+        net.gradients(xd.data_ptr(), td.data_ptr(), torch.zeros_like(md).data_ptr(), n)
+    net.close()
+
+
+@pytest.mark.parametrize("n", [25, 130])
+def test_walks_of_several_slabs_match_fp64(n, require_gpu):
+    """Batches whose slabs (six a sample) exceed the CTAs of the kernels, so
+    that a CTA walks several: output, loss and gradients against the network
+    in FP64, with the bounds of the oracle test (BF16 weights and activations,
+    2^-9 each, through four layers)."""
+    import torch
+    conv = torch.nn.functional.conv3d
+    g = torch.Generator(device="cpu").manual_seed(n)
+    x, t = (torch.randn((n, S, S, S), generator=g).cuda() for _ in range(2))
+    m = (torch.rand((n, S, S, S), generator=g) < 0.5).float().cuda()
+    net = fac.CNN(max_batch=n, seed=9)
+    ws = [torch.from_numpy(w).cuda().double().reshape(s).requires_grad_() for w, s in
+          zip(net.get_weights(), [(27, 1, 16), (27, 16, 16), (27, 16, 16), (27, 16, 1)])]
+    y_ref, loss_ref = [], 0.0
+    for b in range(0, n, 10):
+        h = x[b:b + 10, None].double()
+        for i, w in enumerate(ws):
+            k = w.reshape(3, 3, 3, w.shape[1], w.shape[2]).permute(4, 3, 0, 1, 2)
+            h = conv(h, k, padding=1)
+            h = torch.relu(h) if i < 3 else h
+        part = (m[b:b + 10].double() * (h[:, 0] - t[b:b + 10].double()) ** 2).sum() / m.double().sum()
+        part.backward()
+        loss_ref += float(part.detach())
+        y_ref.append(h[:, 0].detach())
+    y = torch.zeros_like(x)
+    net.forward(x.data_ptr(), n, y.data_ptr())
+    assert rel(y.cpu().numpy(), torch.cat(y_ref).cpu().numpy()) < 1e-2
+    loss, gs = net.gradients(x.data_ptr(), t.data_ptr(), m.data_ptr(), n)
+    assert abs(loss - loss_ref) <= 1e-2 * loss_ref
+    for gr, w in zip(gs, ws):
+        r = w.grad.cpu().numpy().reshape(gr.shape)
+        assert rel(gr, r) < 3e-2, rel(gr, r)
+    net.close()
