@@ -508,6 +508,26 @@ struct fac_ctx {
    DevArray<WorkReg> d_work_regs;
    DevArray<long long> sweeps_call, sweeps_coarse;
    DevArray<double2> norm_acc;
+   // results of the last reduction in pinned memory the GPU writes: per
+   // problem the two sums, and the device error flag
+   struct HostBack {
+      double2 *acc = nullptr;
+      int *err = nullptr;
+      void alloc(int np)
+      {
+         free();
+         CUDA_CHECK(cudaHostAlloc((void **)&acc, np * sizeof(double2) + sizeof(int),
+                                  cudaHostAllocDefault));
+         err = reinterpret_cast<int *>(acc + np);
+         *err = 0;
+      }
+      void free()
+      {
+         if (acc) cudaFreeHost(acc);
+         acc = nullptr;
+      }
+      ~HostBack() { free(); }
+   } back;
    std::vector<std::vector<double>> hist;  // per problem residual history
 
    void drop_graph()
@@ -2480,6 +2500,7 @@ void initialize(fac_ctx *c)
    c->sweeps_call.alloc(np);
    c->sweeps_coarse.alloc(np);
    c->norm_acc.alloc(np);
+   if (!g_dry) c->back.alloc(np);
    c->hist.assign(np, {});
    if (!g_dry) {
       CUDA_CHECK(cudaMemsetAsync(c->sweeps_coarse.p, 0, np * sizeof(long long), c->stream));
@@ -2718,31 +2739,34 @@ void prolong_correct(fac_ctx *c, int fid_src, int fid_dst, int dest_ln)
    CUDA_CHECK(cudaGetLastError());
 }
 
-void rms_norm_launch(fac_ctx *c, int fid)
+// One reduction over all levels of fields x (and y) into norm_acc and, on the
+// host, into back (valid once the stream has drained).
+void reduce_launch(fac_ctx *c, int mode, int fid_x, int fid_y)
 {
-   const int np = nprob(c);
-   CUDA_CHECK(cudaMemsetAsync(c->norm_acc.p, 0, np * sizeof(double2), c->stream));
-   const int g = field_ghost(fid);
+   ReduceLevels lv;
+   lv.n = c->nlev;
+   lv.first[0] = 0;
    for (int ln = 0; ln < c->nlev; ++ln) {
       LevelState &L = c->L[ln];
-      launch_norm(c->stream, c->dim, (int)L.cell_chunks.size(), L.d_patches.p, L.d_cell_chunks.p,
-                  field_ptr(L, fid), g, L.w.p, L.norm_partial.p, L.d_prob_cell_chunk_begin.p, np,
-                  c->norm_acc.p);
+      lv.level[ln] = {L.d_patches.p, L.d_cell_chunks.p, field_ptr(L, fid_x), field_ptr(L, fid_y),
+                      L.w.p, L.norm_partial.p, L.d_prob_cell_chunk_begin.p, field_ghost(fid_x),
+                      field_ghost(fid_y)};
+      lv.first[ln + 1] = lv.first[ln] + (int)L.cell_chunks.size();
    }
+   launch_reduce(c->stream, c->dim, mode, lv, nprob(c), c->norm_acc.p, c->back.acc, c->kerr.p,
+                 c->back.err);
 }
+
+void rms_norm_launch(fac_ctx *c, int fid) { reduce_launch(c, kReduceNorm, fid, fid); }
 
 void rms_norm_read(fac_ctx *c, std::vector<double> &out)
 {
    const int np = nprob(c);
-   std::vector<double2> acc(np);
-   CUDA_CHECK(cudaMemcpyAsync(acc.data(), c->norm_acc.p, np * sizeof(double2),
-                              cudaMemcpyDeviceToHost, c->stream));
-   int kerr = 0;
-   CUDA_CHECK(cudaMemcpyAsync(&kerr, c->kerr.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
    CUDA_CHECK(cudaStreamSynchronize(c->stream));
-   if (kerr)
+   if (*c->back.err)
       throw FacError(FAC_ERR_CUDA, "a bounded wait of a staged colour pass ran out (device error "
                                    "flag; fac_clear_device_error resets it)");
+   const double2 *acc = c->back.acc;
    out.resize(np);
    for (int p = 0; p < np; ++p) {
       const double num = std::sqrt(acc[p].x);
@@ -3504,11 +3528,7 @@ void fgmres_solve(fac_ctx *c, int m, int *converged, int *iterations, double *re
    rms_norm(c, FAC_F, fnorm);
    {
       // sum of the weights per problem (the RMS norm's denominator)
-      std::vector<double2> acc(np);
-      CUDA_CHECK(cudaMemcpyAsync(acc.data(), c->norm_acc.p, np * sizeof(double2),
-                                 cudaMemcpyDeviceToHost, c->stream));
-      CUDA_CHECK(cudaStreamSynchronize(c->stream));
-      for (int p = 0; p < np; ++p) wsum[p] = acc[p].y;
+      for (int p = 0; p < np; ++p) wsum[p] = c->back.acc[p].y;
    }
    std::vector<double> eff(np);
    for (int p = 0; p < np; ++p) {
@@ -4019,25 +4039,13 @@ void vec_all_active(fac_ctx *c)
    }
 }
 
-std::vector<double2> vec_reduce(fac_ctx *c, int mode, int fid_x, int fid_y)
+const double2 *vec_reduce(fac_ctx *c, int mode, int fid_x, int fid_y)
 {
    vec_all_active(c);
-   const int np = nprob(c);
-   const int gx = field_ghost(fid_x), gy = field_ghost(fid_y);
-   CUDA_CHECK(cudaMemsetAsync(c->norm_acc.p, 0, np * sizeof(double2), c->stream));
-   for (int ln = 0; ln < c->nlev; ++ln) {
-      LevelState &L = c->L[ln];
-      launch_vec_reduce(c->stream, c->dim, mode, (int)L.cell_chunks.size(), L.d_patches.p,
-                        L.d_cell_chunks.p, field_ptr(L, fid_x), gx, field_ptr(L, fid_y), gy,
-                        L.w.p, L.norm_partial.p, L.d_prob_cell_chunk_begin.p, np,
-                        c->norm_acc.p);
-   }
+   reduce_launch(c, mode, fid_x, fid_y);
    CUDA_CHECK(cudaGetLastError());
-   std::vector<double2> acc(np);
-   CUDA_CHECK(cudaMemcpyAsync(acc.data(), c->norm_acc.p, np * sizeof(double2),
-                              cudaMemcpyDeviceToHost, c->stream));
    CUDA_CHECK(cudaStreamSynchronize(c->stream));
-   return acc;
+   return c->back.acc;
 }
 
 }  // namespace
@@ -4047,7 +4055,7 @@ int fac_vec_dot(fac_ctx *ctx, int fid_x, int fid_y, double *dots)
    return guarded([&] {
       check_ops(ctx);
       if (!dots) throw FacError(FAC_ERR_ARG, "null output");
-      const std::vector<double2> acc = vec_reduce(ctx, 0, fid_x, fid_y);
+      const double2 *acc = vec_reduce(ctx, kReduceDot, fid_x, fid_y);
       for (int p = 0; p < nprob(ctx); ++p) dots[p] = acc[p].x;
    });
 }
@@ -4057,7 +4065,7 @@ int fac_vec_l2_norm(fac_ctx *ctx, int fid, double *norms)
    return guarded([&] {
       check_ops(ctx);
       if (!norms) throw FacError(FAC_ERR_ARG, "null output");
-      const std::vector<double2> acc = vec_reduce(ctx, 0, fid, fid);
+      const double2 *acc = vec_reduce(ctx, kReduceDot, fid, fid);
       for (int p = 0; p < nprob(ctx); ++p) norms[p] = std::sqrt(acc[p].x);
    });
 }
@@ -4067,7 +4075,7 @@ int fac_vec_max_norm(fac_ctx *ctx, int fid, double *norms)
    return guarded([&] {
       check_ops(ctx);
       if (!norms) throw FacError(FAC_ERR_ARG, "null output");
-      const std::vector<double2> acc = vec_reduce(ctx, 1, fid, fid);
+      const double2 *acc = vec_reduce(ctx, kReduceMax, fid, fid);
       for (int p = 0; p < nprob(ctx); ++p) norms[p] = acc[p].x;
    });
 }
@@ -4081,7 +4089,7 @@ int fac_vec_linear_sum(fac_ctx *ctx, int fid_z, const double *a, int fid_x, cons
       if (fid_z == FAC_W) throw FacError(FAC_ERR_ARG, "the weights are not a vector");
       vec_all_active(ctx);
       const int np = nprob(ctx);
-      ctx->vec_coef.alloc(2 * (size_t)np);
+      if (ctx->vec_coef.n != 2 * (size_t)np) ctx->vec_coef.alloc(2 * (size_t)np);
       CUDA_CHECK(cudaMemcpyAsync(ctx->vec_coef.p, a, np * sizeof(double),
                                  cudaMemcpyHostToDevice, ctx->stream));
       CUDA_CHECK(cudaMemcpyAsync(ctx->vec_coef.p + np, b, np * sizeof(double),
@@ -4114,7 +4122,7 @@ int fac_tag_gradient(fac_ctx *ctx, int fid, int ln, double threshold, long long 
       const int np = nprob(ctx);
       if (L.tag.n != (size_t)std::max<long long>(1, L.n0))
          L.tag.alloc(std::max<long long>(1, L.n0));
-      ctx->tag_counts.alloc(np);
+      if (ctx->tag_counts.n != (size_t)np) ctx->tag_counts.alloc(np);
       CUDA_CHECK(cudaMemsetAsync(ctx->tag_counts.p, 0, np * sizeof(unsigned long long),
                                  ctx->stream));
       launch_adaption_tags(ctx->stream, ctx->dim, (int)L.cell_chunks.size(), L.d_patches.p,

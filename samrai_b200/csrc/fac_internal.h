@@ -11,6 +11,8 @@
 
 #include <cstdint>
 
+#include <vector_types.h>
+
 namespace samrai_b200 {
 
 constexpr int kMaxLevels = 8;
@@ -410,6 +412,26 @@ struct UnitCopy {
    int nbytes;
    int dst_off;
    int total;
+};
+
+// A composite-vector reduction over all levels (k_reduce_partial): per level
+// its chunks ({patch, first cell, cells, own index}; first[l] counts those of the
+// levels below l), the fields with their ghost widths, the partial sums per
+// chunk and each problem's first chunk.
+enum ReduceMode : int { kReduceDot = 0, kReduceMax = 1, kReduceNorm = 2 };
+constexpr int kReducePer = kChunk / 256;  // cells of a chunk per thread
+struct ReduceLevel {
+   const PatchDesc *patches;
+   const Chunk *chunks;
+   const double *x, *y, *w;
+   double2 *partial;
+   const int *begin;
+   int xg, yg;
+};
+struct ReduceLevels {
+   int n;
+   int first[kMaxLevels + 1];
+   ReduceLevel level[kMaxLevels];
 };
 
 // Coarsest-level solve by one thread-block cluster per problem

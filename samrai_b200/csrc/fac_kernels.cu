@@ -1103,141 +1103,136 @@ k_add_interior(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ 
    }
 }
 
-// Weighted sums sum(w x^2), sum(w) per chunk.
-template <int DIM>
-__global__ void __launch_bounds__(kThreads)
-k_norm_partial(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ chunks, int nwork,
-               const double *__restrict__ x, int xg, const double *__restrict__ w,
-               double2 *__restrict__ partial)
+// The tree over 256 values by one warp (lane tid): values t + 128, + 64, + 32
+// added pairwise, then lanes; the same additions as a tree over the block.
+template <int MODE>
+__device__ __forceinline__ void reduce_tree(const double *rs, const double *rv, int tid,
+                                            double2 *__restrict__ out)
 {
-   WORK_LOOP(ch) {
-      const PatchDesc p = patches[ch.patch];
-      const int nx = p.hi[0] - p.lo[0] + 1;
-      const int ny = p.hi[1] - p.lo[1] + 1;
-      const long long xoff = xg ? p.off1 : p.off0;
-      double sd = 0.0, sv = 0.0;
-      if (!xg) {
-         // ghost-0 field: the same linear index as the weights
-         for (int t = threadIdx.x; t < ch.count; t += blockDim.x) {
-            const long long c = p.off0 + ch.begin + t;
-            const double xv = x[c];
-            const double wv = w[c];
-            sd += xv * xv * wv;
-            sv += wv;
-         }
-      } else {
-         for (int t = threadIdx.x; t < ch.count; t += blockDim.x) {
-            const int lin = ch.begin + t;
-            int ci, cj, ck;
-            patch_cell(p, lin, nx, ny, ci, cj, ck);
-            const int i = p.lo[0] + ci;
-            const int j = p.lo[1] + cj;
-            const int k = DIM == 3 ? p.lo[2] + ck : 0;
-            const double xv = x[cidx<DIM>(p, xoff, xg, i, j, k)];
-            const double wv = w[p.off0 + lin];
-            sd += xv * xv * wv;
-            sv += wv;
-         }
-      }
-      __shared__ double rs[kThreads], rv[kThreads];
-      rs[threadIdx.x] = sd;
-      rv[threadIdx.x] = sv;
-      __syncthreads();
-      for (int o = kThreads / 2; o > 0; o >>= 1) {
-         if ((int)threadIdx.x < o) {
-            rs[threadIdx.x] += rs[threadIdx.x + o];
-            rv[threadIdx.x] += rv[threadIdx.x + o];
-         }
-         __syncthreads();
-      }
-      if (threadIdx.x == 0) partial[ch.aux] = make_double2(rs[0], rv[0]);
-      __syncthreads();  // shared memory is reused by the next chunk
+   static_assert(kThreads == 256, "eight values a lane");
+   auto op = [](double a, double b) { return MODE == kReduceMax ? fmax(a, b) : a + b; };
+   double a[4], b[4];
+#pragma unroll
+   for (int q = 0; q < 4; ++q) {
+      a[q] = op(rs[tid + 32 * q], rs[tid + 32 * q + 128]);
+      b[q] = rv[tid + 32 * q] + rv[tid + 32 * q + 128];
    }
+   double sd = op(op(a[0], a[2]), op(a[1], a[3]));
+   double sv = (b[0] + b[2]) + (b[1] + b[3]);
+   for (int o = 16; o > 0; o >>= 1) {
+      sd = op(sd, __shfl_down_sync(0xffffffffu, sd, o));
+      sv += __shfl_down_sync(0xffffffffu, sv, o);
+   }
+   if (tid == 0) *out = make_double2(sd, sv);
 }
 
-// Composite-vector reductions (SAMRAIVectorReal::dot and maxNorm with
-// control volumes, SAMRAIVectorReal.C:821-960 over HierarchyCellDataOpsReal
-// dot/maxNorm, HierarchyCellDataOpsReal.C:877-1036): MODE 0, per chunk the
-// sum of w x y (and of w); MODE 1, the largest |x| over cells with w > 0.
-// Interior cells of fields of any ghost width.
+// Composite-vector reductions over every level in one launch
+// (SAMRAIVectorReal::RMSNorm, dot and maxNorm with control volumes,
+// SAMRAIVectorReal.C:821-960 over HierarchyCellDataOpsReal, HierarchyCellDataOpsReal.C:
+// 877-1036): MODE kReduceDot, per chunk the sums of w x y and of w;
+// kReduceMax, the largest |x| over cells with w > 0; kReduceNorm, the sums of
+// w x x and of w.  Interior cells of fields of any ghost width.  Each thread's
+// cells in the order t, t + 256, ...; then the tree that adds thread t + o to
+// thread t for o = 128, 64, .. 1, its last six steps in one warp while the
+// others load their next chunk.
+//
+// Small vectors are bound by launches and the way back to the host, so a
+// reduction is two launches whatever the number of levels, the second of which
+// writes into pinned memory: dot, two norms and the maximum of an 8192-cell
+// vector 80 us, 164 with two launches a level, the tree over the block and
+// copies to pageable memory; of 2.8 million cells 130 us and 253.
 template <int DIM, int MODE>
 __global__ void __launch_bounds__(kThreads)
-k_vec_partial(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ chunks, int nwork,
-              const double *__restrict__ x, int xg, const double *__restrict__ y, int yg,
-              const double *__restrict__ w, double2 *__restrict__ partial)
+k_reduce_partial(ReduceLevels lv)
 {
-   WORK_LOOP(ch) {
-      const PatchDesc p = patches[ch.patch];
-      const int nx = p.hi[0] - p.lo[0] + 1;
-      const int ny = p.hi[1] - p.lo[1] + 1;
-      const long long xoff = xg ? p.off1 : p.off0, yoff = yg ? p.off1 : p.off0;
-      double sd = 0.0, sv = 0.0;
-      for (int t = threadIdx.x; t < ch.count; t += blockDim.x) {
+   __shared__ double rs[2][kThreads], rv[2][kThreads];
+   int buf = 0;
+   const int tid = threadIdx.x;
+   for (int w0 = blockIdx.x; w0 < lv.first[lv.n]; w0 += gridDim.x) {
+      int l = 0;
+      while (w0 >= lv.first[l + 1]) ++l;
+      const ReduceLevel &L = lv.level[l];
+      const Chunk ch = L.chunks[w0 - lv.first[l]];
+      if (ch.patch < 0) continue;  // end of the level's active chunks
+      const PatchDesc &p = L.patches[ch.patch];
+      const int nx = p.hi[0] - p.lo[0] + 1, ny = p.hi[1] - p.lo[1] + 1;
+      const double *x = L.x + (L.xg ? p.off1 : p.off0);
+      const double *y = L.y + (L.yg ? p.off1 : p.off0);
+      const double *w = L.w + p.off0;
+      double xv[kReducePer], yv[kReducePer], wv[kReducePer];
+#pragma unroll
+      for (int q = 0; q < kReducePer; ++q) {
+         const int t = tid + q * kThreads;
+         wv[q] = xv[q] = yv[q] = 0.0;
+         if (t >= ch.count) continue;
          const int lin = ch.begin + t;
-         int ci, cj, ck;
-         patch_cell(p, lin, nx, ny, ci, cj, ck);
-         const int i = p.lo[0] + ci;
-         const int j = p.lo[1] + cj;
-         const int k = DIM == 3 ? p.lo[2] + ck : 0;
-         const double xv = x[cidx<DIM>(p, xoff, xg, i, j, k)];
-         const double wv = w[p.off0 + lin];
-         if (MODE == 0) {
-            const double yv = y[cidx<DIM>(p, yoff, yg, i, j, k)];
-            sd += xv * yv * wv;
-            sv += wv;
-         } else if (wv > 0.0) {
-            sd = fmax(sd, fabs(xv));
+         long long cx = lin, c1 = lin;
+         if (L.xg || L.yg) {
+            int ci, cj, ck;
+            patch_cell(p, lin, nx, ny, ci, cj, ck);
+            c1 = ci + 1 + (long long)(nx + 2) * (cj + 1 + (DIM == 3 ? (long long)(ny + 2) * (ck + 1) : 0));
+         }
+         if (L.xg) cx = c1;
+         wv[q] = w[lin];
+         xv[q] = x[cx];
+         if (MODE == kReduceDot) yv[q] = y[L.yg ? c1 : lin];
+      }
+      double sd = 0.0, sv = 0.0;
+#pragma unroll
+      for (int q = 0; q < kReducePer; ++q) {
+         if (tid + q * kThreads >= ch.count) break;
+         if (MODE == kReduceMax) {
+            if (wv[q] > 0.0) sd = fmax(sd, fabs(xv[q]));
+         } else {
+            sd += xv[q] * (MODE == kReduceDot ? yv[q] : xv[q]) * wv[q];
+            sv += wv[q];
          }
       }
-      __shared__ double rs[kThreads], rv[kThreads];
-      rs[threadIdx.x] = sd;
-      rv[threadIdx.x] = sv;
+      rs[buf][tid] = sd;
+      rv[buf][tid] = sv;
       __syncthreads();
-      for (int o = kThreads / 2; o > 0; o >>= 1) {
-         if ((int)threadIdx.x < o) {
-            rs[threadIdx.x] = MODE == 0 ? rs[threadIdx.x] + rs[threadIdx.x + o]
-                                        : fmax(rs[threadIdx.x], rs[threadIdx.x + o]);
-            rv[threadIdx.x] += rv[threadIdx.x + o];
-         }
-         __syncthreads();
-      }
-      if (threadIdx.x == 0) partial[ch.aux] = make_double2(rs[0], rv[0]);
-      __syncthreads();
+      if (tid < 32) reduce_tree<MODE>(rs[buf], rv[buf], tid, L.partial + ch.aux);
+      // the other buffer was read before this chunk's barrier
+      buf ^= 1;
    }
 }
 
-// Per problem: the partials of its chunks in chunk order, added to (MODE 0)
-// or maxed into (MODE 1) acc[prob]; levels in level order by the caller.
+// Per problem: each level's partials in chunk order (thread-strided, the same
+// tree), the levels added in level order; to acc[prob] and to the host (pinned
+// memory), with the device error flag.  A warp per level.
 template <int MODE>
-__global__ void k_vec_reduce(const double2 *__restrict__ partial,
-                             const int *__restrict__ prob_chunk_begin, int nprob,
-                             double2 *__restrict__ acc)
+__global__ void __launch_bounds__(kThreads)
+k_reduce_levels(ReduceLevels lv, double2 *__restrict__ acc, double2 *__restrict__ host,
+                const int *__restrict__ err, int *__restrict__ host_err)
 {
-   const int pr = blockIdx.x;
-   if (pr >= nprob) return;
-   const int b = prob_chunk_begin[pr], e = prob_chunk_begin[pr + 1];
-   __shared__ double rs[kThreads], rv[kThreads];
-   double sd = 0.0, sv = 0.0;
-   for (int c = b + threadIdx.x; c < e; c += blockDim.x) {
-      sd = MODE == 0 ? sd + partial[c].x : fmax(sd, partial[c].x);
-      sv += partial[c].y;
-   }
-   rs[threadIdx.x] = sd;
-   rv[threadIdx.x] = sv;
-   __syncthreads();
-   for (int o = kThreads / 2; o > 0; o >>= 1) {
-      if ((int)threadIdx.x < o) {
-         rs[threadIdx.x] = MODE == 0 ? rs[threadIdx.x] + rs[threadIdx.x + o]
-                                     : fmax(rs[threadIdx.x], rs[threadIdx.x + o]);
-         rv[threadIdx.x] += rv[threadIdx.x + o];
+   __shared__ double rs[kMaxLevels][kThreads], rv[kMaxLevels][kThreads];
+   __shared__ double2 sum[kMaxLevels];
+   const int pr = blockIdx.x, tid = threadIdx.x;
+   for (int l = 0; l < lv.n; ++l) {
+      const int b = lv.level[l].begin[pr], e = lv.level[l].begin[pr + 1];
+      const double2 *partial = lv.level[l].partial;
+      double sd = 0.0, sv = 0.0;
+      for (int c = b + tid; c < e; c += kThreads) {
+         const double2 v = partial[c];
+         sd = MODE == kReduceMax ? fmax(sd, v.x) : sd + v.x;
+         sv += v.y;
       }
-      __syncthreads();
+      rs[l][tid] = sd;
+      rv[l][tid] = sv;
    }
-   if (threadIdx.x == 0) {
-      double2 a = acc[pr];
-      a.x = MODE == 0 ? a.x + rs[0] : fmax(a.x, rs[0]);
-      a.y += rv[0];
+   __syncthreads();
+   const int warp = tid >> 5;
+   if (warp < lv.n) reduce_tree<MODE>(rs[warp], rv[warp], tid & 31, sum + warp);
+   __syncthreads();
+   if (tid == 0) {
+      double2 a = make_double2(0.0, 0.0);
+      for (int l = 0; l < lv.n; ++l) {
+         a.x = MODE == kReduceMax ? fmax(a.x, sum[l].x) : a.x + sum[l].x;
+         a.y += sum[l].y;
+      }
       acc[pr] = a;
+      host[pr] = a;
+      if (pr == 0) *host_err = *err;
    }
 }
 
@@ -2349,39 +2344,34 @@ void launch_convert(cudaStream_t s, const S *src, D *dst, long long n)
    k_convert<S, D><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(src, dst, n);
 }
 
-void launch_norm(cudaStream_t s, int dim, int nchunks, const PatchDesc *patches,
-                 const Chunk *chunks, const double *x, int xg, const double *w,
-                 double2 *partial, const int *prob_chunk_begin, int nprob, double2 *acc)
+void launch_reduce(cudaStream_t s, int dim, int mode, const ReduceLevels &lv, int nprob,
+                   double2 *acc, double2 *host, const int *err, int *host_err)
 {
-   if (nchunks <= 0) return;
-   g_launches.fetch_add(2, std::memory_order_relaxed);
-   if (dim == 2)
-      k_norm_partial<2><<<work_grid(k_norm_partial<2>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, x, xg, w, partial);
-   else
-      k_norm_partial<3><<<work_grid(k_norm_partial<3>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, x, xg, w, partial);
-   k_norm_reduce<<<nprob, kThreads, 0, s>>>(partial, prob_chunk_begin, nprob, acc);
-}
-
-void launch_vec_reduce(cudaStream_t s, int dim, int mode, int nchunks, const PatchDesc *patches,
-                       const Chunk *chunks, const double *x, int xg, const double *y, int yg,
-                       const double *w, double2 *partial, const int *prob_chunk_begin,
-                       int nprob, double2 *acc)
-{
-   if (nchunks <= 0) return;
-   g_launches.fetch_add(2, std::memory_order_relaxed);
-#define VP(D, M)                                                                          \
-   k_vec_partial<D, M><<<work_grid(k_vec_partial<D, M>, nchunks), kThreads, 0, s>>>(       \
-      patches, chunks, nchunks, x, xg, y, yg, w, partial)
-   if (dim == 2) {
-      if (mode == 0) VP(2, 0);
-      else VP(2, 1);
+   const int n = lv.first[lv.n];
+   g_launches.fetch_add(n > 0 ? 2 : 1, std::memory_order_relaxed);
+#define VP(D, M) k_reduce_partial<D, M><<<work_grid(k_reduce_partial<D, M>, n), kThreads, 0, s>>>(lv)
+#define VR(M) k_reduce_levels<M><<<nprob, kThreads, 0, s>>>(lv, acc, host, err, host_err)
+   if (mode == kReduceDot) {
+      if (n > 0) {
+         if (dim == 2) VP(2, kReduceDot);
+         else VP(3, kReduceDot);
+      }
+      VR(kReduceDot);
+   } else if (mode == kReduceMax) {
+      if (n > 0) {
+         if (dim == 2) VP(2, kReduceMax);
+         else VP(3, kReduceMax);
+      }
+      VR(kReduceMax);
    } else {
-      if (mode == 0) VP(3, 0);
-      else VP(3, 1);
+      if (n > 0) {
+         if (dim == 2) VP(2, kReduceNorm);
+         else VP(3, kReduceNorm);
+      }
+      VR(kReduceNorm);
    }
 #undef VP
-   if (mode == 0) k_vec_reduce<0><<<nprob, kThreads, 0, s>>>(partial, prob_chunk_begin, nprob, acc);
-   else k_vec_reduce<1><<<nprob, kThreads, 0, s>>>(partial, prob_chunk_begin, nprob, acc);
+#undef VR
 }
 
 void launch_vec_lincomb(cudaStream_t s, int dim, int nchunks, const PatchDesc *patches,
