@@ -10,6 +10,7 @@
 // one patch or one transaction), so patches of uneven size share the grid.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 #include <mutex>
@@ -100,7 +101,7 @@ k_fill(const FillItem *__restrict__ items, const Chunk *__restrict__ chunks, int
        const int *__restrict__ active)
 {
    WORK_LOOP(ch) {
-      for (int t = threadIdx.x; t < ch.count; t += blockDim.x) {
+      ELEMENT_LOOP(t, ch) {
          int lin;
          const FillItem &it = items[chunk_item(ch, prefix, t, lin)];
          if (active && !active[it.prob]) continue;
@@ -112,14 +113,15 @@ k_fill(const FillItem *__restrict__ items, const Chunk *__restrict__ chunks, int
 // Ghost fill from a gather list: element e sets dst[to[e]] from the same
 // level (from[e] >= 0) or from the coarser level's element -from[e] - 1
 // (constant refine), when its problem prob[e] is active.  A flat launch:
-// each thread of the first nblk blocks has kFillPer elements in flight (its
+// each thread of the first nblk blocks has PER elements in flight (its
 // index loads, then its value loads).  The blocks after them walk the
-// physical-boundary items of the same fill.
+// physical-boundary items of the same fill, bcsub blocks to a chunk.
+// PER = 4 where the list fills the GPU that way, 1 below (kFillPer).
 constexpr int kFillPer = 4;
 
-template <class T>
+template <class T, int PER>
 __global__ void __launch_bounds__(kThreads)
-k_fill_gather(long long n, int nblk, const unsigned *__restrict__ to,
+k_fill_gather(long long n, int nblk, int bcsub, const unsigned *__restrict__ to,
               const int *__restrict__ from, const unsigned short *__restrict__ prob,
               const FillItem *__restrict__ bc_items, const Chunk *__restrict__ bc_chunks, int nbc,
               const int *__restrict__ bc_prefix, T *__restrict__ dst,
@@ -127,12 +129,12 @@ k_fill_gather(long long n, int nblk, const unsigned *__restrict__ to,
               BcCoefs bc, const int *__restrict__ active)
 {
    if ((int)blockIdx.x < nblk) {
-      const long long e0 = (long long)blockIdx.x * (kThreads * kFillPer) + threadIdx.x;
-      unsigned d[kFillPer];
-      int sx[kFillPer];
-      bool on[kFillPer];
+      const long long e0 = (long long)blockIdx.x * (kThreads * PER) + threadIdx.x;
+      unsigned d[PER];
+      int sx[PER];
+      bool on[PER];
 #pragma unroll
-      for (int q = 0; q < kFillPer; ++q) {
+      for (int q = 0; q < PER; ++q) {
          const long long e = e0 + q * kThreads;
          on[q] = e < n;
          d[q] = 0u;
@@ -143,19 +145,19 @@ k_fill_gather(long long n, int nblk, const unsigned *__restrict__ to,
             if (active) on[q] = active[prob[e]] != 0;
          }
       }
-      T v[kFillPer];
+      T v[PER];
 #pragma unroll
-      for (int q = 0; q < kFillPer; ++q)
+      for (int q = 0; q < PER; ++q)
          if (on[q]) v[q] = sx[q] >= 0 ? src_same[sx[q]] : src_coarse[-(sx[q] + 1)];
 #pragma unroll
-      for (int q = 0; q < kFillPer; ++q)
+      for (int q = 0; q < PER; ++q)
          if (on[q]) dst[d[q]] = v[q];
       return;
    }
-   for (int w = (int)blockIdx.x - nblk; w < nbc; w += (int)gridDim.x - nblk) {
-      const Chunk ch = bc_chunks[w];
+   for (int w = (int)blockIdx.x - nblk; w < nbc * bcsub; w += (int)gridDim.x - nblk) {
+      const Chunk ch = bc_chunks[w / bcsub];
       if (ch.patch < 0) break;
-      for (int t = threadIdx.x; t < ch.count; t += blockDim.x) {
+      for (int t = threadIdx.x + w % bcsub * kThreads; t < ch.count; t += bcsub * kThreads) {
          int lin;
          const FillItem &it = bc_items[chunk_item(ch, bc_prefix, t, lin)];
          if (active && !active[it.prob]) continue;
@@ -360,7 +362,7 @@ k_rbgs(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ chunks, 
       const T dzi = DIM == 3 ? one / (T)p.dx[2] : (T)0;
       const bool has_cf = (p.flags & 1) != 0;
       double maxres = 0.0;
-      for (int t = threadIdx.x; t < ch.count; t += blockDim.x)
+      ELEMENT_LOOP(t, ch)
          rb_slot<DIM, DVAR, CKIND, T, FUSED>(p, ch.begin + t, nx, ny, hx, dxi, dyi, dzi, has_cf, u,
                                              f, dside, cfield, cfflux, cfmask, offset, dconst,
                                              cconst, facemap, bc, maxres);
@@ -487,7 +489,7 @@ k_flux_cells(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ ch
       const int gx = nx + 2, gxy = (nx + 2) * (ny + 2);
       const TU *up = u + p.off1;
       const double dai[3] = {1. / p.dx[0], 1. / p.dx[1], DIM == 3 ? 1. / p.dx[2] : 0.0};
-      for (int t = threadIdx.x; t < ch.count; t += blockDim.x) {
+      ELEMENT_LOOP(t, ch) {
          const int lin = ch.begin + t;
          int li, lj, lk;
          patch_cell(p, lin, nx, ny, li, lj, lk);
@@ -564,7 +566,7 @@ k_residual(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ chun
       const double dzi = DIM == 3 ? 1. / p.dx[2] : 0.0;
       const double *fx = flux + p.offs[0], *fy = flux + p.offs[1];
       const double *fz = DIM == 3 ? flux + p.offs[2] : nullptr;
-      for (int t = threadIdx.x; t < ch.count; t += blockDim.x) {
+      ELEMENT_LOOP(t, ch) {
          const int lin = ch.begin + t;
          int li, lj, lk;
          patch_cell(p, lin, nx, ny, li, lj, lk);
@@ -721,7 +723,7 @@ k_residual_fused(const PatchDesc *__restrict__ patches, const Chunk *__restrict_
       const int nx = p.hi[0] - p.lo[0] + 1;
       const int ny = p.hi[1] - p.lo[1] + 1;
       const double dai[3] = {1. / p.dx[0], 1. / p.dx[1], DIM == 3 ? 1. / p.dx[2] : 0.0};
-      for (int t = threadIdx.x; t < ch.count; t += blockDim.x) {
+      ELEMENT_LOOP(t, ch) {
          const int lin = ch.begin + t;
          int li, lj, lk;
          patch_cell(p, lin, nx, ny, li, lj, lk);
@@ -772,7 +774,7 @@ k_flux_coarsen(const FluxCoarsenItem *__restrict__ items, const Chunk *__restric
                double *__restrict__ flux_coarse, const int *__restrict__ run)
 {
    WORK_LOOP(ch) {
-      for (int t = threadIdx.x; t < ch.count; t += blockDim.x) {
+      ELEMENT_LOOP(t, ch) {
          int lin;
          const FluxCoarsenItem &it = items[chunk_item(ch, prefix, t, lin)];
          if (run && !run[it.prob]) continue;
@@ -837,7 +839,7 @@ k_restrict(const RestrictItem *__restrict__ items, const Chunk *__restrict__ chu
            double *__restrict__ dst, int dst_g, const int *__restrict__ run)
 {
    WORK_LOOP(ch) {
-      for (int t = threadIdx.x; t < ch.count; t += blockDim.x) {
+      ELEMENT_LOOP(t, ch) {
          int lin;
          const RestrictItem &it = items[chunk_item(ch, prefix, t, lin)];
          if (run && !run[it.prob]) continue;
@@ -932,7 +934,7 @@ k_prolong_add(const ProlongItem *__restrict__ items, const Chunk *__restrict__ c
          }
       }
       __syncthreads();
-      for (int t = threadIdx.x; t < ch.count; t += blockDim.x) {
+      ELEMENT_LOOP(t, ch) {
          int lin;
          const ProlongItem &it = items[chunk_item(ch, prefix, t, lin)];
          const PatchDesc &p = fine[it.fine_patch];
@@ -1017,7 +1019,7 @@ k_prolong_add_r2(const ProlongItem *__restrict__ items, const Chunk *__restrict_
          s_sh[a][ir] = sh;
       }
       __syncthreads();
-      for (int t = threadIdx.x; t < ch.count; t += blockDim.x) {
+      ELEMENT_LOOP(t, ch) {
          int lin;
          const ProlongItem &it = items[chunk_item(ch, prefix, t, lin)];
          const PatchDesc &p = fine[it.fine_patch];
@@ -1090,7 +1092,7 @@ k_add_interior(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ 
       if (run && !run[p.prob]) continue;
       const int nx = p.hi[0] - p.lo[0] + 1;
       const int ny = p.hi[1] - p.lo[1] + 1;
-      for (int t = threadIdx.x; t < ch.count; t += blockDim.x) {
+      ELEMENT_LOOP(t, ch) {
          const int lin = ch.begin + t;
          int ci, cj, ck;
          patch_cell(p, lin, nx, ny, ci, cj, ck);
@@ -1249,7 +1251,7 @@ k_vec_lincomb(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ c
       const int nx = p.hi[0] - p.lo[0] + 1;
       const int ny = p.hi[1] - p.lo[1] + 1;
       const double ap = a[p.prob], bp = b[p.prob];
-      for (int t = threadIdx.x; t < ch.count; t += blockDim.x) {
+      ELEMENT_LOOP(t, ch) {
          const int lin = ch.begin + t;
          int ci, cj, ck;
          patch_cell(p, lin, nx, ny, ci, cj, ck);
@@ -1357,7 +1359,7 @@ k_g0_to_g1(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ chun
       const PatchDesc p = patches[ch.patch];
       const int nx = p.hi[0] - p.lo[0] + 1;
       const int ny = p.hi[1] - p.lo[1] + 1;
-      for (int t = threadIdx.x; t < ch.count; t += blockDim.x) {
+      ELEMENT_LOOP(t, ch) {
          const int lin = ch.begin + t;
          int ci, cj, ck;
          patch_cell(p, lin, nx, ny, ci, cj, ck);
@@ -1433,7 +1435,7 @@ k_scatter_samples(const PatchDesc *__restrict__ patches, const Chunk *__restrict
       const int ny = p.hi[1] - p.lo[1] + 1;
       const long long S3 = (long long)S * S * S;
       const double f = scale[ch.patch] * p.dx[0] * p.dx[0];
-      for (int t = threadIdx.x; t < ch.count; t += blockDim.x) {
+      ELEMENT_LOOP(t, ch) {
          const int lin = ch.begin + t;
          const int a = lin % nx;
          const int r = lin / nx;
@@ -1504,7 +1506,7 @@ k_apply_alpha(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ c
       if (al == 0.0) continue;
       const int nx = p.hi[0] - p.lo[0] + 1;
       const int ny = p.hi[1] - p.lo[1] + 1;
-      for (int t = threadIdx.x; t < ch.count; t += blockDim.x) {
+      ELEMENT_LOOP(t, ch) {
          const int lin = ch.begin + t;
          int ci, cj, ck;
          patch_cell(p, lin, nx, ny, ci, cj, ck);
@@ -1780,7 +1782,7 @@ k_g1_to_g0(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ chun
       const PatchDesc &p = patches[ch.patch];
       const int nx = p.hi[0] - p.lo[0] + 1;
       const int ny = p.hi[1] - p.lo[1] + 1;
-      for (int t = threadIdx.x; t < ch.count; t += blockDim.x) {
+      ELEMENT_LOOP(t, ch) {
          const int lin = ch.begin + t;
          int ci, cj, ck;
          patch_cell(p, lin, nx, ny, ci, cj, ck);
@@ -1808,7 +1810,7 @@ k_add_combination(const PatchDesc *__restrict__ patches, const Chunk *__restrict
       const int nx = p.hi[0] - p.lo[0] + 1;
       const int ny = p.hi[1] - p.lo[1] + 1;
       const double *yp = y + (long long)p.prob * K;
-      for (int t = threadIdx.x; t < ch.count; t += blockDim.x) {
+      ELEMENT_LOOP(t, ch) {
          const int lin = ch.begin + t;
          int ci, cj, ck;
          patch_cell(p, lin, nx, ny, ci, cj, ck);
@@ -1946,10 +1948,10 @@ void launch_g1_to_g0(cudaStream_t s, int dim, int nchunks, const PatchDesc *patc
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
    if (dim == 2)
-      k_g1_to_g0<2, TS><<<work_grid(k_g1_to_g0<2, TS>, nchunks), kThreads, 0, s>>>(
+      k_g1_to_g0<2, TS><<<split_grid(k_g1_to_g0<2, TS>, nchunks), kThreads, 0, s>>>(
          patches, chunks, nchunks, src, dst, add ? 1 : 0, scale, dst1);
    else
-      k_g1_to_g0<3, TS><<<work_grid(k_g1_to_g0<3, TS>, nchunks), kThreads, 0, s>>>(
+      k_g1_to_g0<3, TS><<<split_grid(k_g1_to_g0<3, TS>, nchunks), kThreads, 0, s>>>(
          patches, chunks, nchunks, src, dst, add ? 1 : 0, scale, dst1);
 }
 template void launch_g1_to_g0<double>(cudaStream_t, int, int, const PatchDesc *, const Chunk *,
@@ -1964,10 +1966,10 @@ void launch_add_combination(cudaStream_t s, int dim, int nchunks, const PatchDes
    if (nchunks <= 0 || K <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
    if (dim == 2)
-      k_add_combination<2><<<work_grid(k_add_combination<2>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, u, Z,
+      k_add_combination<2><<<split_grid(k_add_combination<2>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, u, Z,
                                                                     zstride, K, y);
    else
-      k_add_combination<3><<<work_grid(k_add_combination<3>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, u, Z,
+      k_add_combination<3><<<split_grid(k_add_combination<3>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, u, Z,
                                                                     zstride, K, y);
 }
 
@@ -1989,7 +1991,7 @@ void launch_fill(cudaStream_t s, const FillItem *items, const Chunk *chunks, int
 {
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
-   k_fill<T><<<work_grid(k_fill<T>, nchunks), kThreads, 0, s>>>(items, chunks, nchunks, prefix, dst, src_same, src_coarse,
+   k_fill<T><<<split_grid(k_fill<T>, nchunks), kThreads, 0, s>>>(items, chunks, nchunks, prefix, dst, src_same, src_coarse,
                                           homogeneous, bc, active);
 }
 
@@ -2000,14 +2002,20 @@ void launch_fill_gather(cudaStream_t s, long long n, const unsigned *to, const i
                         const T *src_same, const T *src_coarse, int homogeneous,
                         const BcCoefs &bc, const int *active)
 {
-   const long long nblk = (n + kThreads * kFillPer - 1) / (kThreads * kFillPer);
-   const int gbc = nbc > 0 ? work_grid(k_fill_gather<T>, nbc) : 0;
+   // one element per thread while that is at most one resident wave
+   const int cap = resident_blocks(reinterpret_cast<const void *>(k_fill_gather<T, 1>));
+   const bool small = n <= (long long)cap * kThreads;
+   const int per = kThreads * (small ? 1 : kFillPer);
+   const long long nblk = (n + per - 1) / per;
+   const int bcsub = element_split(nbc, cap);
+   const long long gbc = nbc > 0 ? std::min((long long)nbc * bcsub, (long long)cap) : 0;
    if (nblk + gbc <= 0) return;
    if (nblk + gbc > (1ll << 31) - 1) throw std::runtime_error("fill gather list too long");
    g_launches.fetch_add(1, std::memory_order_relaxed);
-   k_fill_gather<T><<<(unsigned)(nblk + gbc), kThreads, 0, s>>>(
-      n, (int)nblk, to, from, prob, bc_items, bc_chunks, nbc, bc_prefix, dst, src_same,
-      src_coarse, homogeneous, bc, active);
+   auto *fn = small ? k_fill_gather<T, 1> : k_fill_gather<T, kFillPer>;
+   fn<<<(unsigned)(nblk + gbc), kThreads, 0, s>>>(n, (int)nblk, bcsub, to, from, prob, bc_items,
+                                                  bc_chunks, nbc, bc_prefix, dst, src_same,
+                                                  src_coarse, homogeneous, bc, active);
 }
 
 template <class T>
@@ -2035,11 +2043,11 @@ static void rbgs_inst(cudaStream_t s, int nchunks, const PatchDesc *patches,
                       const long long *facemap, const BcCoefs &bc)
 {
    if (facemap)
-      k_rbgs<DIM, DVAR, CK, T, true><<<work_grid(k_rbgs<DIM, DVAR, CK, T, true>, nchunks), kThreads, 0, s>>>(
+      k_rbgs<DIM, DVAR, CK, T, true><<<split_grid(k_rbgs<DIM, DVAR, CK, T, true>, nchunks), kThreads, 0, s>>>(
          patches, chunks, nchunks, u, f, dside, cfield, cfflux, cfmask, offset, (T)dconst, (T)cconst,
          maxres, run, facemap, bc);
    else
-      k_rbgs<DIM, DVAR, CK, T, false><<<work_grid(k_rbgs<DIM, DVAR, CK, T, false>, nchunks), kThreads, 0, s>>>(
+      k_rbgs<DIM, DVAR, CK, T, false><<<split_grid(k_rbgs<DIM, DVAR, CK, T, false>, nchunks), kThreads, 0, s>>>(
          patches, chunks, nchunks, u, f, dside, cfield, cfflux, cfmask, offset, (T)dconst, (T)cconst,
          maxres, run, facemap, bc);
 }
@@ -2128,7 +2136,7 @@ void launch_flux_cells(cudaStream_t s, int dim, const PoissonSpec &spec, int nch
       w.longwt[a] = longwt[a];
    }
 #define FC(D, V)                                                                            \
-   k_flux_cells<D, V, TU><<<work_grid(k_flux_cells<D, V, TU>, nchunks), kThreads, 0, s>>>(                          \
+   k_flux_cells<D, V, TU><<<split_grid(k_flux_cells<D, V, TU>, nchunks), kThreads, 0, s>>>(                          \
       patches, cell_chunks, nchunks, u, dside, spec.d_const, cfmask, w, ratio_dev, flux, run)
    if (dim == 2) {
       if (spec.d_variable) FC(2, true);
@@ -2172,7 +2180,7 @@ void launch_residual_fused(cudaStream_t s, int dim, const PoissonSpec &spec, int
       w.longwt[a] = longwt[a];
    }
 #define RF(D, V, C)                                                                         \
-   k_residual_fused<D, V, C, TU><<<work_grid(k_residual_fused<D, V, C, TU>, nchunks), kThreads, 0, s>>>(                   \
+   k_residual_fused<D, V, C, TU><<<split_grid(k_residual_fused<D, V, C, TU>, nchunks), kThreads, 0, s>>>(                   \
       patches, chunks, nchunks, u, dside, spec.d_const, cfmask, w, ratio_dev, fcmask, fcflux, \
       f, cfield, spec.c_const, res, oflux, run)
    if (dim == 2) {
@@ -2253,7 +2261,7 @@ void launch_residual(cudaStream_t s, int dim, const PoissonSpec &spec, int nchun
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
 #define RS(D, C)                                                                         \
-   k_residual<D, C, TU><<<work_grid(k_residual<D, C, TU>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, u, f, flux, cfield, \
+   k_residual<D, C, TU><<<split_grid(k_residual<D, C, TU>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, u, f, flux, cfield, \
                                                      spec.c_const, res, oflux, run)
    if (dim == 2) {
       if (spec.c_kind == 2) RS(2, 2);
@@ -2274,7 +2282,7 @@ void launch_flux_coarsen(cudaStream_t s, const FluxCoarsenItem *items, const Chu
 {
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
-   k_flux_coarsen<<<work_grid(k_flux_coarsen, nchunks), kThreads, 0, s>>>(items, chunks, nchunks, prefix, fine,
+   k_flux_coarsen<<<split_grid(k_flux_coarsen, nchunks), kThreads, 0, s>>>(items, chunks, nchunks, prefix, fine,
                                                           coarse, oflux_fine, flux_coarse, run);
 }
 
@@ -2286,10 +2294,10 @@ void launch_restrict(cudaStream_t s, int dim, const RestrictItem *items, const C
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
    if (dim == 2)
-      k_restrict<2><<<work_grid(k_restrict<2>, nchunks), kThreads, 0, s>>>(items, chunks, nchunks, prefix, fine,
+      k_restrict<2><<<split_grid(k_restrict<2>, nchunks), kThreads, 0, s>>>(items, chunks, nchunks, prefix, fine,
                                                             coarse, src, src_g, dst, dst_g, run);
    else
-      k_restrict<3><<<work_grid(k_restrict<3>, nchunks), kThreads, 0, s>>>(items, chunks, nchunks, prefix, fine,
+      k_restrict<3><<<split_grid(k_restrict<3>, nchunks), kThreads, 0, s>>>(items, chunks, nchunks, prefix, fine,
                                                             coarse, src, src_g, dst, dst_g, run);
 }
 
@@ -2301,10 +2309,10 @@ void launch_prolong_add(cudaStream_t s, int dim, const ProlongItem *items, const
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
    if (dim == 2)
-      k_prolong_add<2, T><<<work_grid(k_prolong_add<2, T>, nchunks), kThreads, 0, s>>>(
+      k_prolong_add<2, T><<<split_grid(k_prolong_add<2, T>, nchunks), kThreads, 0, s>>>(
          items, chunks, nchunks, prefix, fine, tmp, dxc_prob, ratio[0], ratio[1], ratio[2], e, run);
    else
-      k_prolong_add<3, T><<<work_grid(k_prolong_add<3, T>, nchunks), kThreads, 0, s>>>(
+      k_prolong_add<3, T><<<split_grid(k_prolong_add<3, T>, nchunks), kThreads, 0, s>>>(
          items, chunks, nchunks, prefix, fine, tmp, dxc_prob, ratio[0], ratio[1], ratio[2], e, run);
 }
 
@@ -2317,10 +2325,10 @@ void launch_prolong_add_r2(cudaStream_t s, int dim, const ProlongItem *items,
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
    if (dim == 2)
-      k_prolong_add_r2<2, T><<<work_grid(k_prolong_add_r2<2, T>, nchunks), kThreads, 0, s>>>(
+      k_prolong_add_r2<2, T><<<split_grid(k_prolong_add_r2<2, T>, nchunks), kThreads, 0, s>>>(
          items, chunks, nchunks, prefix, fine, tmp, dxc_prob, e, run);
    else
-      k_prolong_add_r2<3, T><<<work_grid(k_prolong_add_r2<3, T>, nchunks), kThreads, 0, s>>>(
+      k_prolong_add_r2<3, T><<<split_grid(k_prolong_add_r2<3, T>, nchunks), kThreads, 0, s>>>(
          items, chunks, nchunks, prefix, fine, tmp, dxc_prob, e, run);
 }
 
@@ -2331,9 +2339,9 @@ void launch_add_interior(cudaStream_t s, int dim, int nchunks, const PatchDesc *
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
    if (dim == 2)
-      k_add_interior<2, T><<<work_grid(k_add_interior<2, T>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, u, e, run);
+      k_add_interior<2, T><<<split_grid(k_add_interior<2, T>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, u, e, run);
    else
-      k_add_interior<3, T><<<work_grid(k_add_interior<3, T>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, u, e, run);
+      k_add_interior<3, T><<<split_grid(k_add_interior<3, T>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, u, e, run);
 }
 
 template <class S, class D>
@@ -2381,10 +2389,10 @@ void launch_vec_lincomb(cudaStream_t s, int dim, int nchunks, const PatchDesc *p
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
    if (dim == 2)
-      k_vec_lincomb<2><<<work_grid(k_vec_lincomb<2>, nchunks), kThreads, 0, s>>>(
+      k_vec_lincomb<2><<<split_grid(k_vec_lincomb<2>, nchunks), kThreads, 0, s>>>(
          patches, chunks, nchunks, z, zg, x, xg, y, yg, a, b);
    else
-      k_vec_lincomb<3><<<work_grid(k_vec_lincomb<3>, nchunks), kThreads, 0, s>>>(
+      k_vec_lincomb<3><<<split_grid(k_vec_lincomb<3>, nchunks), kThreads, 0, s>>>(
          patches, chunks, nchunks, z, zg, x, xg, y, yg, a, b);
 }
 
@@ -2409,8 +2417,8 @@ void launch_g0_to_g1(cudaStream_t s, int dim, int nchunks, const PatchDesc *patc
 {
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
-   if (dim == 2) k_g0_to_g1<2><<<work_grid(k_g0_to_g1<2>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, src, dst);
-   else k_g0_to_g1<3><<<work_grid(k_g0_to_g1<3>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, src, dst);
+   if (dim == 2) k_g0_to_g1<2><<<split_grid(k_g0_to_g1<2>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, src, dst);
+   else k_g0_to_g1<3><<<split_grid(k_g0_to_g1<3>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, src, dst);
 }
 
 void launch_patch_rms(cudaStream_t s, int dim, int npatch, const PatchDesc *patches,
@@ -2440,9 +2448,9 @@ void launch_scatter_samples(cudaStream_t s, int dim, int nchunks, const PatchDes
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
    if (dim == 2)
-      k_scatter_samples<2><<<work_grid(k_scatter_samples<2>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, y, scale, S, dst);
+      k_scatter_samples<2><<<split_grid(k_scatter_samples<2>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, y, scale, S, dst);
    else
-      k_scatter_samples<3><<<work_grid(k_scatter_samples<3>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, y, scale, S, dst);
+      k_scatter_samples<3><<<split_grid(k_scatter_samples<3>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, y, scale, S, dst);
 }
 
 void launch_dot_pair(cudaStream_t s, int dim, int nchunks, const PatchDesc *patches,
@@ -2472,9 +2480,9 @@ void launch_apply_alpha(cudaStream_t s, int dim, int nchunks, const PatchDesc *p
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
    if (dim == 2)
-      k_apply_alpha<2><<<work_grid(k_apply_alpha<2>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, alpha, u, e, r, r2);
+      k_apply_alpha<2><<<split_grid(k_apply_alpha<2>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, alpha, u, e, r, r2);
    else
-      k_apply_alpha<3><<<work_grid(k_apply_alpha<3>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, alpha, u, e, r, r2);
+      k_apply_alpha<3><<<split_grid(k_apply_alpha<3>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, alpha, u, e, r, r2);
 }
 
 void launch_gather(cudaStream_t s, const long long *idx, long long n, const double *src,
