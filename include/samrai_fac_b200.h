@@ -331,7 +331,7 @@ int fac_trace_read(fac_ctx *ctx, char *buf, int cap, int *len);
 int fac_kernel_launches(long long *n);
 /* Record CUDA events around every red-black colour pass (kind 0 FP64,
  * kind 2 FP32), ghost fill (kind 1 FP64, kind 3 FP32) and FGMRES vector
- * operation (kind 4 multi-dot, kind 5 linear combination; per level) from
+ * operation (kind 4 multi-dot, kind 5 linear combination; all levels) from
  * now on; clears earlier records.  Bytes count only problems still
  * iterating. */
 int fac_profile_enable(fac_ctx *ctx, int on);

@@ -366,6 +366,7 @@ struct LevelState {
    std::vector<int> prob_span_begin;
    DevArray<int> d_prob_span_begin;
    std::vector<double> cells_prob;  // ghost-0 cells per problem
+   bool covered = false;            // every cell lies under a finer level
    DevArray<double2> norm_partial;
 
    ItemList<FillItem> fill_nc, fill_wc;   // ghost fill without / with coarser level
@@ -447,7 +448,26 @@ struct fac_ctx {
    cudaGraphExec_t prec_exec = nullptr, apply_exec = nullptr;
    long long prec_launches = 0, apply_launches = 0;
    int kry_m = 0;
-   DevArray<double> kry_dots, kry_coef, kry_a;
+   DevArray<double> kry_coef;
+   std::vector<double> kry_cells_prob;  // cells of the levels the vectors live on
+   // pinned: results the vector kernels write, and two buffers their scalars
+   // are copied from
+   struct KryHost {
+      double *dots = nullptr, *coef[2] = {nullptr, nullptr};
+      void alloc(size_t n)
+      {
+         free();
+         CUDA_CHECK(cudaHostAlloc((void **)&dots, 3 * n * sizeof(double), cudaHostAllocDefault));
+         coef[0] = dots + n;
+         coef[1] = coef[0] + n;
+      }
+      void free()
+      {
+         if (dots) cudaFreeHost(dots);
+         dots = nullptr;
+      }
+      ~KryHost() { free(); }
+   } kry_host;
    DevArray<double> vec_coef;  // per-problem scalars of fac_vec_linear_sum
    DevArray<unsigned long long> tag_counts;  // per-problem tag counts
    // clustering scratch, grown as needed and kept between calls
@@ -2121,6 +2141,7 @@ void compute_weights_host(fac_ctx *c)
             }
          }
       }
+      L.covered = L.n0 > 0 && std::all_of(w.begin(), w.end(), [](double v) { return v == 0.0; });
       CUDA_CHECK(cudaMemcpyAsync(L.w.p, w.data(), L.n0 * sizeof(double), cudaMemcpyHostToDevice,
                                  c->stream));
    }
@@ -3275,9 +3296,13 @@ void kry_alloc(fac_ctx *c, int m)
       // finite contents: slots a problem did not reach enter x += Z y with y = 0
       CUDA_CHECK(cudaMemsetAsync(L.kry.p, 0, L.kry.n * sizeof(double), c->stream));
    }
-   c->kry_dots.alloc((size_t)np * (m + 1));
-   c->kry_coef.alloc((size_t)np * (m + 1));
-   c->kry_a.alloc(np);
+   // a problem's scalar and up to m + 1 coefficients
+   c->kry_coef.alloc((size_t)np * (m + 2));
+   c->kry_host.alloc((size_t)np * (m + 2));
+   c->kry_cells_prob.assign(np, 0.0);
+   for (int ln = 0; ln < c->nlev; ++ln)
+      for (int p = 0; p < np && !c->L[ln].covered; ++p)
+         c->kry_cells_prob[p] += c->L[ln].cells_prob[p];
    c->kry_m = m;
 }
 
@@ -3293,28 +3318,62 @@ double *kry_field(fac_ctx *c, int ln, int field)
    return nullptr;
 }
 
+// Operands of a vector operation on every level with uncovered cells.  The
+// others -- a coarse extension's, and every level a finer one covers -- take no
+// part: their weights are 0, and what a vector holds there is overwritten by the
+// restriction of finer values before anything reads it.
+KryLevels kry_levels(fac_ctx *c, int outslot, int xslot, int vslot, int xfield, int x2_field)
+{
+   KryLevels lv;
+   lv.n = 0;
+   lv.first[0] = 0;
+   for (int ln = 0; ln < c->nlev; ++ln) {
+      LevelState &L = c->L[ln];
+      if (L.covered) continue;
+      double *x = xfield != kNoField ? kry_field(c, ln, xfield) : kry_vec(c, ln, xslot);
+      lv.level[lv.n] = {L.d_span_chunks.p, L.w.p, x, kry_vec(c, ln, vslot),
+                        kry_vec(c, ln, outslot),
+                        x2_field != kNoField ? kry_field(c, ln, x2_field) : nullptr,
+                        std::max<long long>(1, L.n0), L.kry_partial.p, L.d_prob_span_begin.p};
+      lv.first[lv.n + 1] = lv.first[lv.n] + (int)L.span_chunks.size();
+      lv.n += 1;
+   }
+   return lv;
+}
+
+// Per-problem scalars a and coefficients (K each) to the device, from pinned
+// buffer `which`; an earlier copy out of the same buffer has been waited for
+// (every use of a buffer is followed by a read-back before its next).
+void kry_scalars(fac_ctx *c, int which, const std::vector<double> &a, int K,
+                 const std::vector<double> &coef)
+{
+   const size_t np = nprob(c);
+   double *h = c->kry_host.coef[which];
+   std::copy(a.begin(), a.begin() + np, h);
+   if (K > 0) std::copy(coef.begin(), coef.begin() + np * K, h + np);
+   CUDA_CHECK(cudaMemcpyAsync(c->kry_coef.p, h, np * (K + 1) * sizeof(double),
+                              cudaMemcpyHostToDevice, c->stream));
+}
+
+void kry_read(fac_ctx *c, int per, std::vector<double> &out)
+{
+   CUDA_CHECK(cudaGetLastError());
+   CUDA_CHECK(cudaStreamSynchronize(c->stream));
+   out.assign(c->kry_host.dots, c->kry_host.dots + (size_t)nprob(c) * per);
+}
+
 // out[p*KT + i] = <x, V_i> (weighted) over all levels, for i < K, x slot
 // xslot or the field xfield; with self_dot KT = K + 1 and entry K is <x, x>
 void kry_dots(fac_ctx *c, int xslot, int vslot, int K, std::vector<double> &out,
               int xfield = kNoField, bool self_dot = false)
 {
    OpTimer ot(c, "kry_dots", -1);
-   const int np = nprob(c);
    const int KT = K + (self_dot ? 1 : 0);
-   CUDA_CHECK(cudaMemsetAsync(c->kry_dots.p, 0, (size_t)np * KT * sizeof(double), c->stream));
-   for (int ln = 0; ln < c->nlev; ++ln) {
-      LevelState &L = c->L[ln];
-      const int pi = prof_begin(c, 4, L.cells_prob, 8.0 * (K + 2));
-      const double *x = xfield != kNoField ? kry_field(c, ln, xfield) : kry_vec(c, ln, xslot);
-      launch_multidot(c->stream, (int)L.span_chunks.size(), L.d_span_chunks.p, L.w.p, x,
-                      kry_vec(c, ln, vslot), std::max<long long>(1, L.n0), K, L.kry_partial.p,
-                      L.d_prob_span_begin.p, np, c->active.p, c->kry_dots.p, self_dot);
-      prof_end(c, pi);
-   }
-   out.resize((size_t)np * KT);
-   CUDA_CHECK(cudaMemcpyAsync(out.data(), c->kry_dots.p, (size_t)np * KT * sizeof(double),
-                              cudaMemcpyDeviceToHost, c->stream));
-   CUDA_CHECK(cudaStreamSynchronize(c->stream));
+   const int pi = prof_begin(c, 4, c->kry_cells_prob, 8.0 * (K + 2));
+   launch_multidot(c->stream, kry_levels(c, xslot, xslot, vslot, xfield, kNoField), K, nprob(c),
+                   c->active.p, c->kry_host.dots, self_dot);
+   prof_end(c, pi);
+   kry_read(c, KT, out);
 }
 
 // V_x = a[p] X + sum_i coef[p*K+i] V_{vslot+i}, X = V_x or the field
@@ -3328,37 +3387,16 @@ void kry_combine(fac_ctx *c, int xslot, const std::vector<double> &a, int vslot,
 {
    OpTimer ot(c, "kry_combine", -1);
    const int np = nprob(c);
-   CUDA_CHECK(cudaMemcpyAsync(c->kry_a.p, a.data(), np * sizeof(double), cudaMemcpyHostToDevice,
-                              c->stream));
-   if (K > 0)
-      CUDA_CHECK(cudaMemcpyAsync(c->kry_coef.p, coef.data(), (size_t)np * K * sizeof(double),
-                                 cudaMemcpyHostToDevice, c->stream));
-   if (norm) CUDA_CHECK(cudaMemsetAsync(c->kry_dots.p, 0, (size_t)np * sizeof(double), c->stream));
-   for (int ln = 0; ln < c->nlev; ++ln) {
-      LevelState &L = c->L[ln];
-      const int pi = prof_begin(c, 5, L.cells_prob, 8.0 * (K + (norm ? 3 : 2)));
-      const double *xin = xin_field != kNoField ? kry_field(c, ln, xin_field) : nullptr;
-      if (norm)
-         launch_combine_norm(c->stream, (int)L.span_chunks.size(), L.d_span_chunks.p,
-                             kry_vec(c, ln, xslot), c->kry_a.p,
-                             K > 0 ? kry_vec(c, ln, vslot) : nullptr,
-                             std::max<long long>(1, L.n0), K, c->kry_coef.p, L.w.p,
-                             L.kry_partial.p, L.d_prob_span_begin.p, np, c->active.p,
-                             c->kry_dots.p, xin);
-      else
-         launch_combine(c->stream, (int)L.span_chunks.size(), L.d_span_chunks.p,
-                        kry_vec(c, ln, xslot), c->kry_a.p,
-                        K > 0 ? kry_vec(c, ln, vslot) : nullptr, std::max<long long>(1, L.n0),
-                        K, c->kry_coef.p, xin,
-                        x2_field != kNoField ? kry_field(c, ln, x2_field) : nullptr);
-      prof_end(c, pi);
-   }
-   if (norm) {
-      norm->resize(np);
-      CUDA_CHECK(cudaMemcpyAsync(norm->data(), c->kry_dots.p, (size_t)np * sizeof(double),
-                                 cudaMemcpyDeviceToHost, c->stream));
-      CUDA_CHECK(cudaStreamSynchronize(c->stream));
-   }
+   kry_scalars(c, 0, a, K, coef);
+   const KryLevels lv = kry_levels(c, xslot, xslot, vslot, xin_field, norm ? kNoField : x2_field);
+   const int pi = prof_begin(c, 5, c->kry_cells_prob, 8.0 * (K + (norm ? 3 : 2)));
+   if (norm)
+      launch_combine_norm(c->stream, lv, c->kry_coef.p, K, c->kry_coef.p + np, np, c->active.p,
+                          c->kry_host.dots);
+   else
+      launch_combine(c->stream, lv, c->kry_coef.p, K, c->kry_coef.p + np);
+   prof_end(c, pi);
+   if (norm) kry_read(c, 1, *norm);
 }
 
 // V_x = a[p] X + sum_i coef[p*K+i] V_{vslot+i} as kry_combine, and
@@ -3373,27 +3411,12 @@ bool kry_combine_dots(fac_ctx *c, int xslot, const std::vector<double> &a, int v
    if (K < 1 || K > kCombineDotsMax) return false;
    OpTimer ot(c, "kry_combine_dots", -1);
    const int np = nprob(c);
-   const int KT = K + 1;
-   CUDA_CHECK(cudaMemcpyAsync(c->kry_a.p, a.data(), np * sizeof(double), cudaMemcpyHostToDevice,
-                              c->stream));
-   CUDA_CHECK(cudaMemcpyAsync(c->kry_coef.p, coef.data(), (size_t)np * K * sizeof(double),
-                              cudaMemcpyHostToDevice, c->stream));
-   CUDA_CHECK(cudaMemsetAsync(c->kry_dots.p, 0, (size_t)np * KT * sizeof(double), c->stream));
-   for (int ln = 0; ln < c->nlev; ++ln) {
-      LevelState &L = c->L[ln];
-      const int pi = prof_begin(c, 5, L.cells_prob, 8.0 * (K + 3));
-      const double *xin = xin_field != kNoField ? kry_field(c, ln, xin_field) : nullptr;
-      launch_combine_dots(c->stream, (int)L.span_chunks.size(), L.d_span_chunks.p,
-                          kry_vec(c, ln, xslot), c->kry_a.p, kry_vec(c, ln, vslot),
-                          std::max<long long>(1, L.n0), K, c->kry_coef.p, L.w.p,
-                          L.kry_partial.p, L.d_prob_span_begin.p, np, c->active.p,
-                          c->kry_dots.p, xin);
-      prof_end(c, pi);
-   }
-   dots.resize((size_t)np * KT);
-   CUDA_CHECK(cudaMemcpyAsync(dots.data(), c->kry_dots.p, (size_t)np * KT * sizeof(double),
-                              cudaMemcpyDeviceToHost, c->stream));
-   CUDA_CHECK(cudaStreamSynchronize(c->stream));
+   kry_scalars(c, 1, a, K, coef);
+   const int pi = prof_begin(c, 5, c->kry_cells_prob, 8.0 * (K + 3));
+   launch_combine_dots(c->stream, kry_levels(c, xslot, xslot, vslot, xin_field, kNoField),
+                       c->kry_coef.p, K, c->kry_coef.p + np, np, c->active.p, c->kry_host.dots);
+   prof_end(c, pi);
+   kry_read(c, K + 1, dots);
    return true;
 }
 
@@ -3607,18 +3630,20 @@ void fgmres_solve(fac_ctx *c, int m, int *converged, int *iterations, double *re
          // operator fills every face ghost of a level before its residual
          // reads it, and edge and corner ghosts are not read
          const bool both = c->mixed && !c->cnn;
+         StoreLevels st;
+         st.n = 0;
+         st.first[0] = 0;
          for (int ln = 0; ln < c->nlev; ++ln) {
             LevelState &L = c->L[ln];
-            if (c->mixed)
-               launch_g1_to_g0<float>(c->stream, c->dim, (int)L.cell_chunks.size(),
-                                      L.d_patches.p, L.d_cell_chunks.p, L.e32.p,
-                                      kry_vec(c, ln, zslot0 + j), false, nullptr,
-                                      both ? L.e.p : nullptr);
-            else
-               launch_g1_to_g0<double>(c->stream, c->dim, (int)L.cell_chunks.size(),
-                                       L.d_patches.p, L.d_cell_chunks.p, L.e.p,
-                                       kry_vec(c, ln, zslot0 + j));
+            if (L.covered) continue;
+            st.level[st.n] = {L.d_patches.p, L.d_cell_chunks.p,
+                              c->mixed ? (const void *)L.e32.p : (const void *)L.e.p,
+                              kry_vec(c, ln, zslot0 + j), both ? L.e.p : nullptr};
+            st.first[st.n + 1] = st.first[st.n] + (int)L.cell_chunks.size();
+            st.n += 1;
          }
+         if (c->mixed) launch_store_levels<float>(c->stream, c->dim, st);
+         else launch_store_levels<double>(c->stream, c->dim, st);
          if (c->cnn) learned_precondition(c, j, zslot0 + j);
          if (!both) {
             zero_field(c, FAC_E);
@@ -3754,7 +3779,7 @@ void fgmres_solve(fac_ctx *c, int m, int *converged, int *iterations, double *re
          } else {
             kry_combine(c, j + 1, a, 0, 0, coef, nullptr, kNoField, FAC_R);
          }
-         set_active(c, act);
+         if (act != c->host_active) set_active(c, act);
          c->host_active = act;
       }
       // x += Z y for every problem of this restart cycle

@@ -434,6 +434,39 @@ struct ReduceLevels {
    ReduceLevel level[kMaxLevels];
 };
 
+// Operands of the Krylov vector kernels on every level that has uncovered
+// cells: its chunks of problem runs ({problem, first cell, cells, own index};
+// first[l] counts those of the levels before), the weights, the vector read
+// (x), the basis V (one vector every vstride elements), the vector written
+// (out, and out2 when not null), partial sums and each problem's first chunk.
+struct KryLevel {
+   const Chunk *chunks;
+   const double *w, *x, *V;
+   double *out, *out2;
+   long long vstride;
+   double *partial;
+   const int *begin;
+};
+struct KryLevels {
+   int n;
+   int first[kMaxLevels + 1];
+   KryLevel level[kMaxLevels];
+};
+
+// Interior copies (k_store_levels) on every such level: ghost-1 source, ghost-0
+// destination and a ghost-1 FP64 one when not null.
+struct StoreLevel {
+   const PatchDesc *patches;
+   const Chunk *chunks;
+   const void *src;
+   double *dst, *dst1;
+};
+struct StoreLevels {
+   int n;
+   int first[kMaxLevels + 1];
+   StoreLevel level[kMaxLevels];
+};
+
 // Coarsest-level solve by one thread-block cluster per problem
 // (fac_coarse.cu): threads of a CTA and the cells of each colour a thread
 // may own (compiled for 1, 2 and 4).

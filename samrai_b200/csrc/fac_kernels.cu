@@ -1553,6 +1553,24 @@ k_compact(const WorkReg *__restrict__ regs, const int *__restrict__ active, int 
 // level, one vector every vstride elements), per problem, deterministic
 // ---------------------------------------------------------------------------
 
+// The Krylov vector kernels run over all levels in one launch: chunk number w_
+// of the levels one after another.  (A launch and a reduction per level, small
+// levels 4 to 10 us each, and read-backs through pageable memory: the multi-dot
+// of a seven-level, 6.9 million cell context took 170 us of launches, 60 here;
+// four mixed FGMRES solves 24.3 ms and 20.8.)
+#define LEVELS_LOOP(ch, L, lv)                                                 \
+   for (int w_ = blockIdx.x, l_ = 0; w_ < lv.first[lv.n]; w_ += gridDim.x)      \
+      if (l_ = level_of(lv.first, w_); true)                                    \
+         if (const auto &L = lv.level[l_]; true)                                \
+            if (const Chunk ch = L.chunks[w_ - lv.first[l_]]; ch.patch >= 0)
+
+__device__ __forceinline__ int level_of(const int *first, int w)
+{
+   int l = 0;
+   while (w >= first[l + 1]) ++l;
+   return l;
+}
+
 // Vectors a multi-dot or combination takes per pass over the cells: their
 // loads are independent, so a thread keeps that many in flight.
 constexpr int kVecBlock = 8;
@@ -1564,13 +1582,14 @@ constexpr int kVecBlock = 8;
 // With SELF, entry K is <x, x>: x taken as one more vector after the K.
 template <bool SELF>
 __global__ void __launch_bounds__(kThreads)
-k_multidot(const Chunk *__restrict__ chunks, int nwork, const double *__restrict__ w,
-           const double *__restrict__ x, const double *__restrict__ V, long long vstride, int K,
-           double *__restrict__ partial)
+k_multidot(KryLevels lv, int K)
 {
    __shared__ double red[kVecBlock][kThreads / 32];
    const int KT = K + (SELF ? 1 : 0);
-   WORK_LOOP(ch) {
+   LEVELS_LOOP(ch, L, lv) {
+      const double *__restrict__ w = L.w, *__restrict__ x = L.x, *__restrict__ V = L.V;
+      const long long vstride = L.vstride;
+      double *__restrict__ partial = L.partial;
       const long long c0 = ch.begin;
       for (int i0 = 0; i0 < KT; i0 += kVecBlock) {
          const int nb = KT - i0 < kVecBlock ? KT - i0 : kVecBlock;
@@ -1607,24 +1626,30 @@ k_multidot(const Chunk *__restrict__ chunks, int nwork, const double *__restrict
    }
 }
 
-// out[p * K + i] += sum of the problem's chunk partials, in chunk order
-__global__ void k_multidot_reduce(const double *__restrict__ partial,
-                                  const int *__restrict__ prob_chunk_begin, int K,
-                                  const int *__restrict__ active, double *__restrict__ out)
+// out[p * K + i] = sum of the problem's chunk partials, level by level in chunk
+// order (0 for a problem that is not active); out is pinned host memory
+__global__ void __launch_bounds__(kThreads)
+k_multidot_reduce(KryLevels lv, int K, const int *__restrict__ active, double *__restrict__ out)
 {
-   const int p = blockIdx.x, i = blockIdx.y;
-   if (active && !active[p]) return;
-   const int b = prob_chunk_begin[p], e = prob_chunk_begin[p + 1];
-   __shared__ double red[kThreads];
-   double sum = 0.0;
-   for (int c = b + threadIdx.x; c < e; c += blockDim.x) sum += partial[(long long)c * K + i];
-   red[threadIdx.x] = sum;
-   __syncthreads();
-   for (int o = kThreads / 2; o > 0; o >>= 1) {
-      if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-      __syncthreads();
+   const int p = blockIdx.x, i = blockIdx.y, tid = threadIdx.x;
+   const bool on = !active || active[p];
+   __shared__ double red[kMaxLevels][kThreads], zero[kThreads];
+   __shared__ double2 sum[kMaxLevels];
+   zero[tid] = 0.0;
+   for (int l = 0; on && l < lv.n; ++l) {
+      const int b = lv.level[l].begin[p], e = lv.level[l].begin[p + 1];
+      double s = 0.0;
+      for (int c = b + tid; c < e; c += kThreads) s += lv.level[l].partial[(long long)c * K + i];
+      red[l][tid] = s;
    }
-   if (threadIdx.x == 0) out[(long long)p * K + i] += red[0];
+   __syncthreads();
+   if (on && (tid >> 5) < lv.n) reduce_tree<kReduceDot>(red[tid >> 5], zero, tid & 31, sum + (tid >> 5));
+   __syncthreads();
+   if (tid == 0) {
+      double s = 0.0;
+      for (int l = 0; on && l < lv.n; ++l) s += sum[l].x;
+      out[(long long)p * K + i] = s;
+   }
 }
 
 // x = a[p] x + sum_i coef[p * K + i] V_i over the chunks of problem runs,
@@ -1633,20 +1658,20 @@ __global__ void k_multidot_reduce(const double *__restrict__ partial,
 // of the new x, accumulated exactly as k_multidot accumulates <x, x> (the
 // same cells per thread in the same order, the same warp tree, warps in
 // order), so the pass that would reread x for its norm is saved.
-// The old x is read from xin (x itself when xin is null) and the new one
-// is also written to x2 when that is not null, so a copy before or after
-// the combination needs no pass of its own; xin and x2 may be the same
-// array (each element is read before it is written, by the same thread).
+// The old x is read from xin and the new one is also written to x2 when that
+// is not null, so a copy before or after the combination needs no pass of its
+// own; x, xin and x2 may be the same array (each element is read before it is
+// written, by the same thread).
 template <bool NORM>
 __global__ void __launch_bounds__(kThreads)
-k_combine(const Chunk *__restrict__ chunks, int nwork, double *x, const double *xin,
-          double *x2, const double *__restrict__ a, const double *__restrict__ V,
-          long long vstride, int K, const double *__restrict__ coef,
-          const double *__restrict__ w, double *__restrict__ partial)
+k_combine(KryLevels lv, const double *__restrict__ a, int K, const double *__restrict__ coef)
 {
-   if (!xin) xin = x;
    __shared__ double red[NORM ? kThreads / 32 : 1];
-   WORK_LOOP(ch) {
+   LEVELS_LOOP(ch, L, lv) {
+      double *x = L.out, *x2 = L.out2;
+      const double *xin = L.x, *__restrict__ V = L.V, *__restrict__ w = L.w;
+      const long long vstride = L.vstride;
+      double *__restrict__ partial = L.partial;
       const double ap = a[ch.patch];
       const double *cp = coef + (long long)ch.patch * K;
       // a problem's trailing zero coefficients add nothing: their vectors
@@ -1701,16 +1726,17 @@ k_combine(const Chunk *__restrict__ chunks, int nwork, double *x, const double *
 // products (K <= KB); the coefficients sit in shared memory.
 template <int KB>
 __global__ void __launch_bounds__(kThreads)
-k_combine_dots(const Chunk *__restrict__ chunks, int nwork, double *x, const double *xin,
-               const double *__restrict__ a, const double *__restrict__ V, long long vstride,
-               int K, const double *__restrict__ coef, const double *__restrict__ w,
-               double *__restrict__ partial)
+k_combine_dots(KryLevels lv, const double *__restrict__ a, int K,
+               const double *__restrict__ coef)
 {
-   if (!xin) xin = x;
    __shared__ double red[KB + 1][kThreads / 32];
    __shared__ double scoef[KB];
    const int KT = K + 1;
-   WORK_LOOP(ch) {
+   LEVELS_LOOP(ch, L, lv) {
+      double *x = L.out;
+      const double *xin = L.x, *__restrict__ V = L.V, *__restrict__ w = L.w;
+      const long long vstride = L.vstride;
+      double *__restrict__ partial = L.partial;
       if ((int)threadIdx.x < K) scoef[threadIdx.x] = coef[(long long)ch.patch * K + threadIdx.x];
       __syncthreads();
       const double ap = a[ch.patch];
@@ -1798,6 +1824,30 @@ k_g1_to_g0(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ chun
    }
 }
 
+// The same without scale over all levels in one launch, blocks per chunk as
+// ELEMENT_LOOP
+template <int DIM, class TS>
+__global__ void __launch_bounds__(kThreads)
+k_store_levels(StoreLevels lv)
+{
+   LEVELS_LOOP(ch, L, lv) {
+      const PatchDesc &p = L.patches[ch.patch];
+      const int nx = p.hi[0] - p.lo[0] + 1, ny = p.hi[1] - p.lo[1] + 1;
+      const TS *src = static_cast<const TS *>(L.src) + p.off1;
+      double *dst = L.dst + p.off0, *dst1 = L.dst1 ? L.dst1 + p.off1 : nullptr;
+      ELEMENT_LOOP(t, ch) {
+         const int lin = ch.begin + t;
+         int ci, cj, ck;
+         patch_cell(p, lin, nx, ny, ci, cj, ck);
+         const long long c1 =
+            ci + 1 + (long long)(nx + 2) * (cj + 1 + (DIM == 3 ? (long long)(ny + 2) * (ck + 1) : 0));
+         const double v = (double)src[c1];
+         dst[lin] = v;
+         if (dst1) dst1[c1] = v;
+      }
+   }
+}
+
 // u interior (ghost-1) += sum_i y[p * K + i] Z_i (ghost-0)
 template <int DIM>
 __global__ void __launch_bounds__(kThreads)
@@ -1867,78 +1917,79 @@ long long kernel_launch_count() { return g_launches.load(); }
 
 void add_kernel_launches(long long n) { g_launches += n; }
 
-void launch_multidot(cudaStream_t s, int nchunks, const Chunk *chunks, const double *w,
-                     const double *x, const double *V, long long vstride, int K,
-                     double *partial, const int *prob_chunk_begin, int nprob, const int *active,
+namespace {
+
+void multidot_reduce(cudaStream_t s, const KryLevels &lv, int KT, int nprob, const int *active,
+                     double *out)
+{
+   g_launches.fetch_add(1, std::memory_order_relaxed);
+   k_multidot_reduce<<<dim3(nprob, KT), kThreads, 0, s>>>(lv, KT, active, out);
+}
+
+}  // namespace
+
+void launch_multidot(cudaStream_t s, const KryLevels &lv, int K, int nprob, const int *active,
                      double *out, bool self_dot)
 {
-   const int KT = K + (self_dot ? 1 : 0);
+   const int KT = K + (self_dot ? 1 : 0), n = lv.first[lv.n];
    if (KT <= 0) return;
-   if (nchunks > 0) {
+   if (n > 0) {
       g_launches.fetch_add(1, std::memory_order_relaxed);
-      if (self_dot)
-         k_multidot<true><<<work_grid(k_multidot<true>, nchunks), kThreads, 0, s>>>(
-            chunks, nchunks, w, x, V, vstride, K, partial);
-      else
-         k_multidot<false><<<work_grid(k_multidot<false>, nchunks), kThreads, 0, s>>>(
-            chunks, nchunks, w, x, V, vstride, K, partial);
+      if (self_dot) k_multidot<true><<<work_grid(k_multidot<true>, n), kThreads, 0, s>>>(lv, K);
+      else k_multidot<false><<<work_grid(k_multidot<false>, n), kThreads, 0, s>>>(lv, K);
    }
-   g_launches.fetch_add(1, std::memory_order_relaxed);
-   k_multidot_reduce<<<dim3(nprob, KT), kThreads, 0, s>>>(partial, prob_chunk_begin, KT, active,
-                                                          out);
+   multidot_reduce(s, lv, KT, nprob, active, out);
 }
 
-void launch_combine(cudaStream_t s, int nchunks, const Chunk *chunks, double *x, const double *a,
-                    const double *V, long long vstride, int K, const double *coef,
-                    const double *xin, double *x2)
+void launch_combine(cudaStream_t s, const KryLevels &lv, const double *a, int K, const double *coef)
 {
-   if (nchunks <= 0) return;
+   const int n = lv.first[lv.n];
+   if (n <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
-   k_combine<false><<<work_grid(k_combine<false>, nchunks), kThreads, 0, s>>>(
-      chunks, nchunks, x, xin, x2, a, V, vstride, K, coef, nullptr, nullptr);
+   k_combine<false><<<work_grid(k_combine<false>, n), kThreads, 0, s>>>(lv, a, K, coef);
 }
 
-void launch_combine_norm(cudaStream_t s, int nchunks, const Chunk *chunks, double *x,
-                         const double *a, const double *V, long long vstride, int K,
-                         const double *coef, const double *w, double *partial,
-                         const int *prob_chunk_begin, int nprob, const int *active, double *out,
-                         const double *xin)
+void launch_combine_norm(cudaStream_t s, const KryLevels &lv, const double *a, int K,
+                         const double *coef, int nprob, const int *active, double *out)
 {
-   if (nchunks > 0) {
+   const int n = lv.first[lv.n];
+   if (n > 0) {
       g_launches.fetch_add(1, std::memory_order_relaxed);
-      k_combine<true><<<work_grid(k_combine<true>, nchunks), kThreads, 0, s>>>(
-         chunks, nchunks, x, xin, nullptr, a, V, vstride, K, coef, w, partial);
+      k_combine<true><<<work_grid(k_combine<true>, n), kThreads, 0, s>>>(lv, a, K, coef);
    }
-   g_launches.fetch_add(1, std::memory_order_relaxed);
-   k_multidot_reduce<<<dim3(nprob, 1), kThreads, 0, s>>>(partial, prob_chunk_begin, 1, active,
-                                                         out);
+   multidot_reduce(s, lv, 1, nprob, active, out);
 }
 
-bool launch_combine_dots(cudaStream_t s, int nchunks, const Chunk *chunks, double *x,
-                         const double *a, const double *V, long long vstride, int K,
-                         const double *coef, const double *w, double *partial,
-                         const int *prob_chunk_begin, int nprob, const int *active, double *out,
-                         const double *xin)
+bool launch_combine_dots(cudaStream_t s, const KryLevels &lv, const double *a, int K,
+                         const double *coef, int nprob, const int *active, double *out)
 {
    if (K < 1 || K > kCombineDotsMax) return false;
-   if (nchunks > 0) {
+   const int n = lv.first[lv.n];
+   if (n > 0) {
       g_launches.fetch_add(1, std::memory_order_relaxed);
       if (K <= 8)
-         k_combine_dots<8><<<work_grid(k_combine_dots<8>, nchunks), kThreads, 0, s>>>(
-            chunks, nchunks, x, xin, a, V, vstride, K, coef, w, partial);
+         k_combine_dots<8><<<work_grid(k_combine_dots<8>, n), kThreads, 0, s>>>(lv, a, K, coef);
       else if (K <= 16)
-         k_combine_dots<16><<<work_grid(k_combine_dots<16>, nchunks), kThreads, 0, s>>>(
-            chunks, nchunks, x, xin, a, V, vstride, K, coef, w, partial);
+         k_combine_dots<16><<<work_grid(k_combine_dots<16>, n), kThreads, 0, s>>>(lv, a, K, coef);
       else
          k_combine_dots<kCombineDotsMax>
-            <<<work_grid(k_combine_dots<kCombineDotsMax>, nchunks), kThreads, 0, s>>>(
-               chunks, nchunks, x, xin, a, V, vstride, K, coef, w, partial);
+            <<<work_grid(k_combine_dots<kCombineDotsMax>, n), kThreads, 0, s>>>(lv, a, K, coef);
    }
-   g_launches.fetch_add(1, std::memory_order_relaxed);
-   k_multidot_reduce<<<dim3(nprob, K + 1), kThreads, 0, s>>>(partial, prob_chunk_begin, K + 1,
-                                                             active, out);
+   multidot_reduce(s, lv, K + 1, nprob, active, out);
    return true;
 }
+
+template <class TS>
+void launch_store_levels(cudaStream_t s, int dim, const StoreLevels &lv)
+{
+   const int n = lv.first[lv.n];
+   if (n <= 0) return;
+   g_launches.fetch_add(1, std::memory_order_relaxed);
+   if (dim == 2) k_store_levels<2, TS><<<split_grid(k_store_levels<2, TS>, n), kThreads, 0, s>>>(lv);
+   else k_store_levels<3, TS><<<split_grid(k_store_levels<3, TS>, n), kThreads, 0, s>>>(lv);
+}
+template void launch_store_levels<double>(cudaStream_t, int, const StoreLevels &);
+template void launch_store_levels<float>(cudaStream_t, int, const StoreLevels &);
 
 template <class TS>
 void launch_g1_to_g0(cudaStream_t s, int dim, int nchunks, const PatchDesc *patches,

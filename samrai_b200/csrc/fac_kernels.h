@@ -63,40 +63,32 @@ void launch_tags_dense(cudaStream_t s, int dim, int nchunks, const PatchDesc *pa
 void launch_br_histogram(cudaStream_t s, int nitems, const BrItem *items, const BrNode *nodes,
                          const unsigned char *dense, int *hist);
 
-// Krylov vector operations on composite vectors: ghost-0 level arrays, one
-// vector every vstride elements; per-problem coefficients; chunks are runs
-// of one problem's cells {problem, first cell, cells, chunk index} (partial
-// is nchunks x K).
-// out[p*KT+i] += sum_w x V_i over problem p's chunks of this level, KT = K
-// (+1 with self_dot: entry K is <x, x>, the same sum as taking x as V_K).
-void launch_multidot(cudaStream_t s, int nchunks, const Chunk *chunks, const double *w,
-                     const double *x, const double *V, long long vstride, int K,
-                     double *partial, const int *prob_chunk_begin, int nprob, const int *active,
+// Krylov vector operations on composite vectors over every level of lv, with
+// per-problem coefficients.
+// out[p*KT+i] = sum w x V_i over problem p, KT = K (+1 with self_dot: entry K
+// is <x, x>, the same sum as taking x as V_K); 0 for problems not active.  out
+// (here and below) is pinned host memory.
+void launch_multidot(cudaStream_t s, const KryLevels &lv, int K, int nprob, const int *active,
                      double *out, bool self_dot = false);
-// x = a[p] xin + sum_i coef[p*K+i] V_i (xin null: x itself), also written
-// to x2 when it is not null
-void launch_combine(cudaStream_t s, int nchunks, const Chunk *chunks, double *x, const double *a,
-                    const double *V, long long vstride, int K, const double *coef,
-                    const double *xin = nullptr, double *x2 = nullptr);
-// The same (without x2), and out[p] += <x, x> (weighted, the new x) over
-// problem p's chunks of this level, equal to launch_multidot(x, x, K = 1).
-void launch_combine_norm(cudaStream_t s, int nchunks, const Chunk *chunks, double *x,
-                         const double *a, const double *V, long long vstride, int K,
-                         const double *coef, const double *w, double *partial,
-                         const int *prob_chunk_begin, int nprob, const int *active, double *out,
-                         const double *xin = nullptr);
+// lv.out = a[p] lv.x + sum_i coef[p*K+i] V_i, also written to lv.out2 when
+// it is not null
+void launch_combine(cudaStream_t s, const KryLevels &lv, const double *a, int K, const double *coef);
+// The same, and out[p] = <lv.out, lv.out> (weighted), equal to launch_multidot
+// of the result with itself, K = 1.
+void launch_combine_norm(cudaStream_t s, const KryLevels &lv, const double *a, int K,
+                         const double *coef, int nprob, const int *active, double *out);
 // Largest K of launch_combine_dots.
 constexpr int kCombineDotsMax = 24;
-// x = a[p] xin + sum_i coef[p*K+i] V_i as launch_combine, and out[p*(K+1)+i]
-// += <x, V_i> for i < K, out[p*(K+1)+K] += <x, x> (weighted, the new x) over
-// problem p's chunks of this level: the numbers of launch_multidot(x, V, K,
-// self_dot) after the combination, from the same pass.  Returns false
-// (nothing launched) unless 1 <= K <= kCombineDotsMax.
-bool launch_combine_dots(cudaStream_t s, int nchunks, const Chunk *chunks, double *x,
-                         const double *a, const double *V, long long vstride, int K,
-                         const double *coef, const double *w, double *partial,
-                         const int *prob_chunk_begin, int nprob, const int *active, double *out,
-                         const double *xin = nullptr);
+// lv.out = a[p] lv.x + sum_i coef[p*K+i] V_i as launch_combine, and
+// out[p*(K+1)+i] = <lv.out, V_i> for i < K, out[p*(K+1)+K] = <lv.out, lv.out>
+// (weighted): the numbers of launch_multidot(lv.out, V, K, self_dot) after the
+// combination, from the same pass.  Returns false (nothing launched) unless
+// 1 <= K <= kCombineDotsMax.
+bool launch_combine_dots(cudaStream_t s, const KryLevels &lv, const double *a, int K,
+                         const double *coef, int nprob, const int *active, double *out);
+// interior of a ghost-1 field (TS) into FP64 ghost-0 and ghost-1 fields
+template <class TS>
+void launch_store_levels(cudaStream_t s, int dim, const StoreLevels &lv);
 // dst (ghost-0) = interior of src (ghost-1), converted to FP64, times
 // scale[problem] when scale is given (with add: dst += it); with dst1 (a
 // ghost-1 FP64 field, not src) the same values also go to its interior
