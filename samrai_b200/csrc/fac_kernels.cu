@@ -100,6 +100,7 @@ k_fill(const FillItem *__restrict__ items, const Chunk *__restrict__ chunks, int
        const T *__restrict__ src_coarse, int homogeneous, BcCoefs bc,
        const int *__restrict__ active)
 {
+   pdl_begin();
    WORK_LOOP(ch) {
       ELEMENT_LOOP(t, ch) {
          int lin;
@@ -128,6 +129,7 @@ k_fill_gather(long long n, int nblk, int bcsub, const unsigned *__restrict__ to,
               const T *__restrict__ src_same, const T *__restrict__ src_coarse, int homogeneous,
               BcCoefs bc, const int *__restrict__ active)
 {
+   pdl_begin();
    if ((int)blockIdx.x < nblk) {
       const long long e0 = (long long)blockIdx.x * (kThreads * PER) + threadIdx.x;
       unsigned d[PER];
@@ -204,6 +206,7 @@ k_cf_flux(const CfFace *__restrict__ faces, int nfaces,
           EwingWeights w, T *__restrict__ cfflux,
           const int *__restrict__ run)
 {
+   pdl_begin();
    const int t = blockIdx.x * blockDim.x + threadIdx.x;
    if (t >= nfaces) return;
    const CfFace cf = faces[t];
@@ -351,6 +354,7 @@ k_rbgs(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ chunks, 
        unsigned long long *__restrict__ maxres_patch, const int *__restrict__ run,
        const long long *__restrict__ facemap, BcCoefs bc)
 {
+   pdl_begin();
    WORK_LOOP(ch) {
       const PatchDesc p = patches[ch.patch];
       if (run && !run[p.prob]) continue;
@@ -396,6 +400,7 @@ k_flux(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ chunks, 
        const int *ratio_to_coarser, double *__restrict__ flux,
        const int *__restrict__ run)
 {
+   pdl_begin();
    WORK_LOOP(ch) {
       const PatchDesc p = patches[ch.patch];
       if (run && !run[p.prob]) continue;
@@ -480,6 +485,7 @@ k_flux_cells(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ ch
              const int *ratio_to_coarser, double *__restrict__ flux,
              const int *__restrict__ run)
 {
+   pdl_begin();
    WORK_LOOP(ch) {
       const PatchDesc &p = patches[ch.patch];
       if (run && !run[p.prob]) continue;
@@ -530,6 +536,7 @@ k_ewing_fix(const CfFace *__restrict__ faces, int nfaces, const PatchDesc *__res
             double dconst, EwingWeights w, double *__restrict__ flux,
             const int *__restrict__ run)
 {
+   pdl_begin();
    const int t = blockIdx.x * blockDim.x + threadIdx.x;
    if (t >= nfaces) return;
    const CfFace cf = faces[t];
@@ -555,6 +562,7 @@ k_residual(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ chun
            double cconst, double *__restrict__ res, double *__restrict__ oflux,
            const int *__restrict__ run)
 {
+   pdl_begin();
    WORK_LOOP(ch) {
       const PatchDesc &p = patches[ch.patch];
       if (run && !run[p.prob]) continue;
@@ -717,6 +725,7 @@ k_residual_fused(const PatchDesc *__restrict__ patches, const Chunk *__restrict_
                  const double *__restrict__ cfield, double cconst, double *__restrict__ res,
                  double *__restrict__ oflux, const int *__restrict__ run)
 {
+   pdl_begin();
    WORK_LOOP(ch) {
       const PatchDesc &p = patches[ch.patch];
       if (run && !run[p.prob]) continue;
@@ -748,6 +757,7 @@ k_residual_cells(const CellRef *__restrict__ cells, int ncells,
                  const double *__restrict__ cfield, double cconst, double *__restrict__ res,
                  double *__restrict__ oflux, const int *__restrict__ run)
 {
+   pdl_begin();
    const int e = blockIdx.x * blockDim.x + threadIdx.x;
    if (e >= ncells) return;
    const CellRef cr = cells[e];
@@ -773,6 +783,7 @@ k_flux_coarsen(const FluxCoarsenItem *__restrict__ items, const Chunk *__restric
                const PatchDesc *__restrict__ coarse, const double *__restrict__ oflux_fine,
                double *__restrict__ flux_coarse, const int *__restrict__ run)
 {
+   pdl_begin();
    WORK_LOOP(ch) {
       ELEMENT_LOOP(t, ch) {
          int lin;
@@ -838,6 +849,7 @@ k_restrict(const RestrictItem *__restrict__ items, const Chunk *__restrict__ chu
            const PatchDesc *__restrict__ coarse, const double *__restrict__ src, int src_g,
            double *__restrict__ dst, int dst_g, const int *__restrict__ run)
 {
+   pdl_begin();
    WORK_LOOP(ch) {
       ELEMENT_LOOP(t, ch) {
          int lin;
@@ -905,6 +917,7 @@ k_prolong_add(const ProlongItem *__restrict__ items, const Chunk *__restrict__ c
               const T *__restrict__ tmp, const double *__restrict__ dxc_prob, int ratio0,
               int ratio1, int ratio2, T *__restrict__ e, const int *__restrict__ run)
 {
+   pdl_begin();
    const T half = (T)0.5, one = (T)1;
    const int r[3] = {ratio0, ratio1, ratio2};
    // per axis and fine offset ir within the coarse cell: the interpolation
@@ -997,6 +1010,7 @@ k_prolong_add_r2(const ProlongItem *__restrict__ items, const Chunk *__restrict_
                  const T *__restrict__ tmp, const double *__restrict__ dxc_prob,
                  T *__restrict__ e, const int *__restrict__ run)
 {
+   pdl_begin();
    const T half = (T)0.5, one = (T)1;
    __shared__ T s_x[3][2];
    __shared__ int s_sh[3][2];
@@ -1087,6 +1101,7 @@ k_add_interior(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ 
                double *__restrict__ u, const T *__restrict__ e,
                const int *__restrict__ run)
 {
+   pdl_begin();
    WORK_LOOP(ch) {
       const PatchDesc p = patches[ch.patch];
       if (run && !run[p.prob]) continue;
@@ -1147,6 +1162,7 @@ template <int DIM, int MODE>
 __global__ void __launch_bounds__(kThreads)
 k_reduce_partial(ReduceLevels lv)
 {
+   pdl_begin();
    __shared__ double rs[2][kThreads], rv[2][kThreads];
    int buf = 0;
    const int tid = threadIdx.x;
@@ -1207,6 +1223,7 @@ __global__ void __launch_bounds__(kThreads)
 k_reduce_levels(ReduceLevels lv, double2 *__restrict__ acc, double2 *__restrict__ host,
                 const int *__restrict__ err, int *__restrict__ host_err)
 {
+   pdl_begin();
    __shared__ double rs[kMaxLevels][kThreads], rv[kMaxLevels][kThreads];
    __shared__ double2 sum[kMaxLevels];
    const int pr = blockIdx.x, tid = threadIdx.x;
@@ -1246,6 +1263,7 @@ k_vec_lincomb(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ c
               double *z, int zg, const double *x, int xg, const double *y, int yg,
               const double *__restrict__ a, const double *__restrict__ b)
 {
+   pdl_begin();
    WORK_LOOP(ch) {
       const PatchDesc p = patches[ch.patch];
       const int nx = p.hi[0] - p.lo[0] + 1;
@@ -1271,6 +1289,7 @@ __global__ void k_norm_reduce(const double2 *__restrict__ partial,
                               const int *__restrict__ prob_chunk_begin, int nprob,
                               double2 *__restrict__ acc)
 {
+   pdl_begin();
    const int pr = blockIdx.x;
    if (pr >= nprob) return;
    const int b = prob_chunk_begin[pr], e = prob_chunk_begin[pr + 1];
@@ -1304,6 +1323,7 @@ __global__ void k_sweep_check(const unsigned long long *__restrict__ red,
                               double tol, int *__restrict__ run,
                               long long *__restrict__ sweeps)
 {
+   pdl_begin();
    const int pr = blockIdx.x * blockDim.x + threadIdx.x;
    if (pr >= nprob) return;
    if (!run[pr]) return;
@@ -1320,6 +1340,7 @@ __global__ void k_sweep_check(const unsigned long long *__restrict__ red,
 template <class S, class D>
 __global__ void k_convert(const S *__restrict__ src, D *__restrict__ dst, long long n)
 {
+   pdl_begin();
    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
    if (t < n) dst[t] = (D)src[t];
 }
@@ -1327,6 +1348,7 @@ __global__ void k_convert(const S *__restrict__ src, D *__restrict__ dst, long l
 __global__ void k_accumulate(const long long *__restrict__ src, long long *__restrict__ dst,
                              int n)
 {
+   pdl_begin();
    const int t = blockIdx.x * blockDim.x + threadIdx.x;
    if (t < n) dst[t] += src[t];
 }
@@ -1334,6 +1356,7 @@ __global__ void k_accumulate(const long long *__restrict__ src, long long *__res
 __global__ void k_gather(const long long *__restrict__ idx, long long n,
                          const double *__restrict__ src, double *__restrict__ dst)
 {
+   pdl_begin();
    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
    if (t < n) dst[t] = src[idx[t]];
 }
@@ -1341,6 +1364,7 @@ __global__ void k_gather(const long long *__restrict__ idx, long long n,
 __global__ void k_scatter(const long long *__restrict__ idx, long long n,
                           const double *__restrict__ src, double *__restrict__ dst)
 {
+   pdl_begin();
    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
    if (t < n) dst[idx[t]] = src[t];
 }
@@ -1355,6 +1379,7 @@ __global__ void __launch_bounds__(kThreads)
 k_g0_to_g1(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ chunks, int nwork,
            const double *__restrict__ src, double *__restrict__ dst)
 {
+   pdl_begin();
    WORK_LOOP(ch) {
       const PatchDesc p = patches[ch.patch];
       const int nx = p.hi[0] - p.lo[0] + 1;
@@ -1376,6 +1401,7 @@ template <int DIM>
 __global__ void k_patch_rms(const PatchDesc *__restrict__ patches, const double *__restrict__ x,
                             double *__restrict__ rms)
 {
+   pdl_begin();
    const PatchDesc p = patches[blockIdx.x];
    const long long n = (long long)(p.hi[0] - p.lo[0] + 1) * (p.hi[1] - p.lo[1] + 1) *
                        (p.hi[2] - p.lo[2] + 1);
@@ -1402,6 +1428,7 @@ __global__ void k_gather_samples(const PatchDesc *__restrict__ patches,
                                  const double *__restrict__ x, const double *__restrict__ scale,
                                  float *__restrict__ out, int S)
 {
+   pdl_begin();
    const int ip = blockIdx.y;
    const PatchDesc p = patches[ip];
    const long long S3 = (long long)S * S * S;
@@ -1429,6 +1456,7 @@ k_scatter_samples(const PatchDesc *__restrict__ patches, const Chunk *__restrict
                   const float *__restrict__ y, const double *__restrict__ scale, int S,
                   double *__restrict__ dst)
 {
+   pdl_begin();
    WORK_LOOP(ch) {
       const PatchDesc p = patches[ch.patch];
       const int nx = p.hi[0] - p.lo[0] + 1;
@@ -1456,6 +1484,7 @@ k_dot_pair(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ chun
            const double *__restrict__ r, const double *__restrict__ r2,
            const double *__restrict__ w, double2 *__restrict__ partial)
 {
+   pdl_begin();
    WORK_LOOP(ch) {
       const PatchDesc p = patches[ch.patch];
       double a = 0.0, b = 0.0;
@@ -1486,6 +1515,7 @@ k_dot_pair(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ chun
 __global__ void k_alpha(const double2 *__restrict__ acc, const int *__restrict__ active,
                         int nprob, double *__restrict__ alpha)
 {
+   pdl_begin();
    const int pr = blockIdx.x * blockDim.x + threadIdx.x;
    if (pr >= nprob) return;
    const double a = acc[pr].x, b = acc[pr].y;
@@ -1500,6 +1530,7 @@ k_apply_alpha(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ c
               const double *__restrict__ e, double *__restrict__ r,
               const double *__restrict__ r2)
 {
+   pdl_begin();
    WORK_LOOP(ch) {
       const PatchDesc p = patches[ch.patch];
       const double al = alpha[p.prob];
@@ -1527,6 +1558,7 @@ k_apply_alpha(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ c
 __global__ void __launch_bounds__(kThreads)
 k_compact(const WorkReg *__restrict__ regs, const int *__restrict__ active, int nprob)
 {
+   pdl_begin();
    const WorkReg r = regs[blockIdx.x];
    const int p = blockIdx.y;
    int before = 0;
@@ -1584,6 +1616,7 @@ template <bool SELF>
 __global__ void __launch_bounds__(kThreads)
 k_multidot(KryLevels lv, int K)
 {
+   pdl_begin();
    __shared__ double red[kVecBlock][kThreads / 32];
    const int KT = K + (SELF ? 1 : 0);
    LEVELS_LOOP(ch, L, lv) {
@@ -1631,6 +1664,7 @@ k_multidot(KryLevels lv, int K)
 __global__ void __launch_bounds__(kThreads)
 k_multidot_reduce(KryLevels lv, int K, const int *__restrict__ active, double *__restrict__ out)
 {
+   pdl_begin();
    const int p = blockIdx.x, i = blockIdx.y, tid = threadIdx.x;
    const bool on = !active || active[p];
    __shared__ double red[kMaxLevels][kThreads], zero[kThreads];
@@ -1666,6 +1700,7 @@ template <bool NORM>
 __global__ void __launch_bounds__(kThreads)
 k_combine(KryLevels lv, const double *__restrict__ a, int K, const double *__restrict__ coef)
 {
+   pdl_begin();
    __shared__ double red[NORM ? kThreads / 32 : 1];
    LEVELS_LOOP(ch, L, lv) {
       double *x = L.out, *x2 = L.out2;
@@ -1729,6 +1764,7 @@ __global__ void __launch_bounds__(kThreads)
 k_combine_dots(KryLevels lv, const double *__restrict__ a, int K,
                const double *__restrict__ coef)
 {
+   pdl_begin();
    __shared__ double red[KB + 1][kThreads / 32];
    __shared__ double scoef[KB];
    const int KT = K + 1;
@@ -1804,6 +1840,7 @@ k_g1_to_g0(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ chun
            const TS *__restrict__ src, double *__restrict__ dst, int add,
            const double *__restrict__ scale, double *__restrict__ dst1)
 {
+   pdl_begin();
    WORK_LOOP(ch) {
       const PatchDesc &p = patches[ch.patch];
       const int nx = p.hi[0] - p.lo[0] + 1;
@@ -1830,6 +1867,7 @@ template <int DIM, class TS>
 __global__ void __launch_bounds__(kThreads)
 k_store_levels(StoreLevels lv)
 {
+   pdl_begin();
    LEVELS_LOOP(ch, L, lv) {
       const PatchDesc &p = L.patches[ch.patch];
       const int nx = p.hi[0] - p.lo[0] + 1, ny = p.hi[1] - p.lo[1] + 1;
@@ -1855,6 +1893,7 @@ k_add_combination(const PatchDesc *__restrict__ patches, const Chunk *__restrict
                   int nwork, double *__restrict__ u, const double *__restrict__ Z,
                   long long zstride, int K, const double *__restrict__ y)
 {
+   pdl_begin();
    WORK_LOOP(ch) {
       const PatchDesc &p = patches[ch.patch];
       const int nx = p.hi[0] - p.lo[0] + 1;
@@ -1923,7 +1962,7 @@ void multidot_reduce(cudaStream_t s, const KryLevels &lv, int KT, int nprob, con
                      double *out)
 {
    g_launches.fetch_add(1, std::memory_order_relaxed);
-   k_multidot_reduce<<<dim3(nprob, KT), kThreads, 0, s>>>(lv, KT, active, out);
+   launch_after(k_multidot_reduce, dim3(nprob, KT), kThreads, 0, s, lv, KT, active, out);
 }
 
 }  // namespace
@@ -1935,8 +1974,8 @@ void launch_multidot(cudaStream_t s, const KryLevels &lv, int K, int nprob, cons
    if (KT <= 0) return;
    if (n > 0) {
       g_launches.fetch_add(1, std::memory_order_relaxed);
-      if (self_dot) k_multidot<true><<<work_grid(k_multidot<true>, n), kThreads, 0, s>>>(lv, K);
-      else k_multidot<false><<<work_grid(k_multidot<false>, n), kThreads, 0, s>>>(lv, K);
+      if (self_dot) launch_after(k_multidot<true>, work_grid(k_multidot<true>, n), kThreads, 0, s, lv, K);
+      else launch_after(k_multidot<false>, work_grid(k_multidot<false>, n), kThreads, 0, s, lv, K);
    }
    multidot_reduce(s, lv, KT, nprob, active, out);
 }
@@ -1946,7 +1985,7 @@ void launch_combine(cudaStream_t s, const KryLevels &lv, const double *a, int K,
    const int n = lv.first[lv.n];
    if (n <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
-   k_combine<false><<<work_grid(k_combine<false>, n), kThreads, 0, s>>>(lv, a, K, coef);
+   launch_after(k_combine<false>, work_grid(k_combine<false>, n), kThreads, 0, s, lv, a, K, coef);
 }
 
 void launch_combine_norm(cudaStream_t s, const KryLevels &lv, const double *a, int K,
@@ -1955,7 +1994,7 @@ void launch_combine_norm(cudaStream_t s, const KryLevels &lv, const double *a, i
    const int n = lv.first[lv.n];
    if (n > 0) {
       g_launches.fetch_add(1, std::memory_order_relaxed);
-      k_combine<true><<<work_grid(k_combine<true>, n), kThreads, 0, s>>>(lv, a, K, coef);
+      launch_after(k_combine<true>, work_grid(k_combine<true>, n), kThreads, 0, s, lv, a, K, coef);
    }
    multidot_reduce(s, lv, 1, nprob, active, out);
 }
@@ -1968,12 +2007,11 @@ bool launch_combine_dots(cudaStream_t s, const KryLevels &lv, const double *a, i
    if (n > 0) {
       g_launches.fetch_add(1, std::memory_order_relaxed);
       if (K <= 8)
-         k_combine_dots<8><<<work_grid(k_combine_dots<8>, n), kThreads, 0, s>>>(lv, a, K, coef);
+         launch_after(k_combine_dots<8>, work_grid(k_combine_dots<8>, n), kThreads, 0, s, lv, a, K, coef);
       else if (K <= 16)
-         k_combine_dots<16><<<work_grid(k_combine_dots<16>, n), kThreads, 0, s>>>(lv, a, K, coef);
+         launch_after(k_combine_dots<16>, work_grid(k_combine_dots<16>, n), kThreads, 0, s, lv, a, K, coef);
       else
-         k_combine_dots<kCombineDotsMax>
-            <<<work_grid(k_combine_dots<kCombineDotsMax>, n), kThreads, 0, s>>>(lv, a, K, coef);
+         launch_after(k_combine_dots<kCombineDotsMax>, work_grid(k_combine_dots<kCombineDotsMax>, n), kThreads, 0, s, lv, a, K, coef);
    }
    multidot_reduce(s, lv, K + 1, nprob, active, out);
    return true;
@@ -1985,8 +2023,8 @@ void launch_store_levels(cudaStream_t s, int dim, const StoreLevels &lv)
    const int n = lv.first[lv.n];
    if (n <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
-   if (dim == 2) k_store_levels<2, TS><<<split_grid(k_store_levels<2, TS>, n), kThreads, 0, s>>>(lv);
-   else k_store_levels<3, TS><<<split_grid(k_store_levels<3, TS>, n), kThreads, 0, s>>>(lv);
+   if (dim == 2) launch_after(k_store_levels<2, TS>, split_grid(k_store_levels<2, TS>, n), kThreads, 0, s, lv);
+   else launch_after(k_store_levels<3, TS>, split_grid(k_store_levels<3, TS>, n), kThreads, 0, s, lv);
 }
 template void launch_store_levels<double>(cudaStream_t, int, const StoreLevels &);
 template void launch_store_levels<float>(cudaStream_t, int, const StoreLevels &);
@@ -1999,11 +2037,9 @@ void launch_g1_to_g0(cudaStream_t s, int dim, int nchunks, const PatchDesc *patc
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
    if (dim == 2)
-      k_g1_to_g0<2, TS><<<split_grid(k_g1_to_g0<2, TS>, nchunks), kThreads, 0, s>>>(
-         patches, chunks, nchunks, src, dst, add ? 1 : 0, scale, dst1);
+      launch_after(k_g1_to_g0<2, TS>, split_grid(k_g1_to_g0<2, TS>, nchunks), kThreads, 0, s, patches, chunks, nchunks, src, dst, add ? 1 : 0, scale, dst1);
    else
-      k_g1_to_g0<3, TS><<<split_grid(k_g1_to_g0<3, TS>, nchunks), kThreads, 0, s>>>(
-         patches, chunks, nchunks, src, dst, add ? 1 : 0, scale, dst1);
+      launch_after(k_g1_to_g0<3, TS>, split_grid(k_g1_to_g0<3, TS>, nchunks), kThreads, 0, s, patches, chunks, nchunks, src, dst, add ? 1 : 0, scale, dst1);
 }
 template void launch_g1_to_g0<double>(cudaStream_t, int, int, const PatchDesc *, const Chunk *,
                                       const double *, double *, bool, const double *, double *);
@@ -2017,10 +2053,10 @@ void launch_add_combination(cudaStream_t s, int dim, int nchunks, const PatchDes
    if (nchunks <= 0 || K <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
    if (dim == 2)
-      k_add_combination<2><<<split_grid(k_add_combination<2>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, u, Z,
+      launch_after(k_add_combination<2>, split_grid(k_add_combination<2>, nchunks), kThreads, 0, s, patches, chunks, nchunks, u, Z,
                                                                     zstride, K, y);
    else
-      k_add_combination<3><<<split_grid(k_add_combination<3>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, u, Z,
+      launch_after(k_add_combination<3>, split_grid(k_add_combination<3>, nchunks), kThreads, 0, s, patches, chunks, nchunks, u, Z,
                                                                     zstride, K, y);
 }
 
@@ -2028,7 +2064,7 @@ void launch_compact(cudaStream_t s, const WorkReg *regs, int nregs, const int *a
 {
    if (nregs <= 0 || nprob <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
-   k_compact<<<dim3(nregs, nprob), kThreads, 0, s>>>(regs, active, nprob);
+   launch_after(k_compact, dim3(nregs, nprob), kThreads, 0, s, regs, active, nprob);
 }
 
 // ---------------------------------------------------------------------------
@@ -2042,7 +2078,7 @@ void launch_fill(cudaStream_t s, const FillItem *items, const Chunk *chunks, int
 {
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
-   k_fill<T><<<split_grid(k_fill<T>, nchunks), kThreads, 0, s>>>(items, chunks, nchunks, prefix, dst, src_same, src_coarse,
+   launch_after(k_fill<T>, split_grid(k_fill<T>, nchunks), kThreads, 0, s, items, chunks, nchunks, prefix, dst, src_same, src_coarse,
                                           homogeneous, bc, active);
 }
 
@@ -2064,7 +2100,7 @@ void launch_fill_gather(cudaStream_t s, long long n, const unsigned *to, const i
    if (nblk + gbc > (1ll << 31) - 1) throw std::runtime_error("fill gather list too long");
    g_launches.fetch_add(1, std::memory_order_relaxed);
    auto *fn = small ? k_fill_gather<T, 1> : k_fill_gather<T, kFillPer>;
-   fn<<<(unsigned)(nblk + gbc), kThreads, 0, s>>>(n, (int)nblk, bcsub, to, from, prob, bc_items,
+   launch_after(fn, (unsigned)(nblk + gbc), kThreads, 0, s, n, (int)nblk, bcsub, to, from, prob, bc_items,
                                                   bc_chunks, nbc, bc_prefix, dst, src_same,
                                                   src_coarse, homogeneous, bc, active);
 }
@@ -2082,7 +2118,7 @@ void launch_cf_flux(cudaStream_t s, const CfFace *faces, int nfaces, const Patch
       w.longwt[a] = longwt[a];
    }
    const int nb = (nfaces + kThreads - 1) / kThreads;
-   k_cf_flux<T><<<nb, kThreads, 0, s>>>(faces, nfaces, patches, u, dside, dvar, (T)dconst, w,
+   launch_after(k_cf_flux<T>, nb, kThreads, 0, s, faces, nfaces, patches, u, dside, dvar, (T)dconst, w,
                                         cfflux, run);
 }
 
@@ -2094,12 +2130,10 @@ static void rbgs_inst(cudaStream_t s, int nchunks, const PatchDesc *patches,
                       const long long *facemap, const BcCoefs &bc)
 {
    if (facemap)
-      k_rbgs<DIM, DVAR, CK, T, true><<<split_grid(k_rbgs<DIM, DVAR, CK, T, true>, nchunks), kThreads, 0, s>>>(
-         patches, chunks, nchunks, u, f, dside, cfield, cfflux, cfmask, offset, (T)dconst, (T)cconst,
+      launch_after(k_rbgs<DIM, DVAR, CK, T, true>, split_grid(k_rbgs<DIM, DVAR, CK, T, true>, nchunks), kThreads, 0, s, patches, chunks, nchunks, u, f, dside, cfield, cfflux, cfmask, offset, (T)dconst, (T)cconst,
          maxres, run, facemap, bc);
    else
-      k_rbgs<DIM, DVAR, CK, T, false><<<split_grid(k_rbgs<DIM, DVAR, CK, T, false>, nchunks), kThreads, 0, s>>>(
-         patches, chunks, nchunks, u, f, dside, cfield, cfflux, cfmask, offset, (T)dconst, (T)cconst,
+      launch_after(k_rbgs<DIM, DVAR, CK, T, false>, split_grid(k_rbgs<DIM, DVAR, CK, T, false>, nchunks), kThreads, 0, s, patches, chunks, nchunks, u, f, dside, cfield, cfflux, cfmask, offset, (T)dconst, (T)cconst,
          maxres, run, facemap, bc);
 }
 
@@ -2154,20 +2188,20 @@ void launch_flux(cudaStream_t s, int dim, const PoissonSpec &spec, int nchunks,
    }
    if (dim == 2) {
       if (spec.d_variable)
-         k_flux<2, true, TU><<<work_grid(k_flux<2, true, TU>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, u, dside,
+         launch_after(k_flux<2, true, TU>, work_grid(k_flux<2, true, TU>, nchunks), kThreads, 0, s, patches, chunks, nchunks, u, dside,
                                                           spec.d_const, cfmask, w, ratio_dev,
                                                           flux, run);
       else
-         k_flux<2, false, TU><<<work_grid(k_flux<2, false, TU>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, u, dside,
+         launch_after(k_flux<2, false, TU>, work_grid(k_flux<2, false, TU>, nchunks), kThreads, 0, s, patches, chunks, nchunks, u, dside,
                                                            spec.d_const, cfmask, w,
                                                            ratio_dev, flux, run);
    } else {
       if (spec.d_variable)
-         k_flux<3, true, TU><<<work_grid(k_flux<3, true, TU>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, u, dside,
+         launch_after(k_flux<3, true, TU>, work_grid(k_flux<3, true, TU>, nchunks), kThreads, 0, s, patches, chunks, nchunks, u, dside,
                                                           spec.d_const, cfmask, w, ratio_dev,
                                                           flux, run);
       else
-         k_flux<3, false, TU><<<work_grid(k_flux<3, false, TU>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, u, dside,
+         launch_after(k_flux<3, false, TU>, work_grid(k_flux<3, false, TU>, nchunks), kThreads, 0, s, patches, chunks, nchunks, u, dside,
                                                            spec.d_const, cfmask, w,
                                                            ratio_dev, flux, run);
    }
@@ -2187,8 +2221,7 @@ void launch_flux_cells(cudaStream_t s, int dim, const PoissonSpec &spec, int nch
       w.longwt[a] = longwt[a];
    }
 #define FC(D, V)                                                                            \
-   k_flux_cells<D, V, TU><<<split_grid(k_flux_cells<D, V, TU>, nchunks), kThreads, 0, s>>>(                          \
-      patches, cell_chunks, nchunks, u, dside, spec.d_const, cfmask, w, ratio_dev, flux, run)
+   launch_after(k_flux_cells<D, V, TU>, split_grid(k_flux_cells<D, V, TU>, nchunks), kThreads, 0, s, patches, cell_chunks, nchunks, u, dside, spec.d_const, cfmask, w, ratio_dev, flux, run)
    if (dim == 2) {
       if (spec.d_variable) FC(2, true);
       else FC(2, false);
@@ -2211,8 +2244,7 @@ void launch_ewing_fix(cudaStream_t s, const CfFace *faces, int nfaces, const Pat
       w.tranwt[a] = tranwt[a];
       w.longwt[a] = longwt[a];
    }
-   k_ewing_fix<TU><<<(nfaces + kThreads - 1) / kThreads, kThreads, 0, s>>>(
-      faces, nfaces, patches, u, dside, dvar, dconst, w, flux, run);
+   launch_after(k_ewing_fix<TU>, (nfaces + kThreads - 1) / kThreads, kThreads, 0, s, faces, nfaces, patches, u, dside, dvar, dconst, w, flux, run);
 }
 
 template <class TU>
@@ -2231,8 +2263,7 @@ void launch_residual_fused(cudaStream_t s, int dim, const PoissonSpec &spec, int
       w.longwt[a] = longwt[a];
    }
 #define RF(D, V, C)                                                                         \
-   k_residual_fused<D, V, C, TU><<<split_grid(k_residual_fused<D, V, C, TU>, nchunks), kThreads, 0, s>>>(                   \
-      patches, chunks, nchunks, u, dside, spec.d_const, cfmask, w, ratio_dev, fcmask, fcflux, \
+   launch_after(k_residual_fused<D, V, C, TU>, split_grid(k_residual_fused<D, V, C, TU>, nchunks), kThreads, 0, s, patches, chunks, nchunks, u, dside, spec.d_const, cfmask, w, ratio_dev, fcmask, fcflux, \
       f, cfield, spec.c_const, res, oflux, run)
    if (dim == 2) {
       if (spec.d_variable) {
@@ -2276,8 +2307,7 @@ void launch_residual_cells(cudaStream_t s, int dim, const PoissonSpec &spec, int
    }
    const int grid = (ncells + kThreads - 1) / kThreads;
 #define RC(D, V, C)                                                                          \
-   k_residual_cells<D, V, C, TU><<<grid, kThreads, 0, s>>>(                                   \
-      cells, ncells, patches, u, dside, spec.d_const, cfmask, w, ratio_to_coarser, fcmask,    \
+   launch_after(k_residual_cells<D, V, C, TU>, grid, kThreads, 0, s, cells, ncells, patches, u, dside, spec.d_const, cfmask, w, ratio_to_coarser, fcmask,    \
       fcflux, f, cfield, spec.c_const, res, oflux, run)
    if (dim == 2) {
       if (spec.d_variable) {
@@ -2312,7 +2342,7 @@ void launch_residual(cudaStream_t s, int dim, const PoissonSpec &spec, int nchun
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
 #define RS(D, C)                                                                         \
-   k_residual<D, C, TU><<<split_grid(k_residual<D, C, TU>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, u, f, flux, cfield, \
+   launch_after(k_residual<D, C, TU>, split_grid(k_residual<D, C, TU>, nchunks), kThreads, 0, s, patches, chunks, nchunks, u, f, flux, cfield, \
                                                      spec.c_const, res, oflux, run)
    if (dim == 2) {
       if (spec.c_kind == 2) RS(2, 2);
@@ -2333,7 +2363,7 @@ void launch_flux_coarsen(cudaStream_t s, const FluxCoarsenItem *items, const Chu
 {
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
-   k_flux_coarsen<<<split_grid(k_flux_coarsen, nchunks), kThreads, 0, s>>>(items, chunks, nchunks, prefix, fine,
+   launch_after(k_flux_coarsen, split_grid(k_flux_coarsen, nchunks), kThreads, 0, s, items, chunks, nchunks, prefix, fine,
                                                           coarse, oflux_fine, flux_coarse, run);
 }
 
@@ -2345,10 +2375,10 @@ void launch_restrict(cudaStream_t s, int dim, const RestrictItem *items, const C
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
    if (dim == 2)
-      k_restrict<2><<<split_grid(k_restrict<2>, nchunks), kThreads, 0, s>>>(items, chunks, nchunks, prefix, fine,
+      launch_after(k_restrict<2>, split_grid(k_restrict<2>, nchunks), kThreads, 0, s, items, chunks, nchunks, prefix, fine,
                                                             coarse, src, src_g, dst, dst_g, run);
    else
-      k_restrict<3><<<split_grid(k_restrict<3>, nchunks), kThreads, 0, s>>>(items, chunks, nchunks, prefix, fine,
+      launch_after(k_restrict<3>, split_grid(k_restrict<3>, nchunks), kThreads, 0, s, items, chunks, nchunks, prefix, fine,
                                                             coarse, src, src_g, dst, dst_g, run);
 }
 
@@ -2360,11 +2390,9 @@ void launch_prolong_add(cudaStream_t s, int dim, const ProlongItem *items, const
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
    if (dim == 2)
-      k_prolong_add<2, T><<<split_grid(k_prolong_add<2, T>, nchunks), kThreads, 0, s>>>(
-         items, chunks, nchunks, prefix, fine, tmp, dxc_prob, ratio[0], ratio[1], ratio[2], e, run);
+      launch_after(k_prolong_add<2, T>, split_grid(k_prolong_add<2, T>, nchunks), kThreads, 0, s, items, chunks, nchunks, prefix, fine, tmp, dxc_prob, ratio[0], ratio[1], ratio[2], e, run);
    else
-      k_prolong_add<3, T><<<split_grid(k_prolong_add<3, T>, nchunks), kThreads, 0, s>>>(
-         items, chunks, nchunks, prefix, fine, tmp, dxc_prob, ratio[0], ratio[1], ratio[2], e, run);
+      launch_after(k_prolong_add<3, T>, split_grid(k_prolong_add<3, T>, nchunks), kThreads, 0, s, items, chunks, nchunks, prefix, fine, tmp, dxc_prob, ratio[0], ratio[1], ratio[2], e, run);
 }
 
 template <class T>
@@ -2376,11 +2404,9 @@ void launch_prolong_add_r2(cudaStream_t s, int dim, const ProlongItem *items,
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
    if (dim == 2)
-      k_prolong_add_r2<2, T><<<split_grid(k_prolong_add_r2<2, T>, nchunks), kThreads, 0, s>>>(
-         items, chunks, nchunks, prefix, fine, tmp, dxc_prob, e, run);
+      launch_after(k_prolong_add_r2<2, T>, split_grid(k_prolong_add_r2<2, T>, nchunks), kThreads, 0, s, items, chunks, nchunks, prefix, fine, tmp, dxc_prob, e, run);
    else
-      k_prolong_add_r2<3, T><<<split_grid(k_prolong_add_r2<3, T>, nchunks), kThreads, 0, s>>>(
-         items, chunks, nchunks, prefix, fine, tmp, dxc_prob, e, run);
+      launch_after(k_prolong_add_r2<3, T>, split_grid(k_prolong_add_r2<3, T>, nchunks), kThreads, 0, s, items, chunks, nchunks, prefix, fine, tmp, dxc_prob, e, run);
 }
 
 template <class T>
@@ -2390,9 +2416,9 @@ void launch_add_interior(cudaStream_t s, int dim, int nchunks, const PatchDesc *
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
    if (dim == 2)
-      k_add_interior<2, T><<<split_grid(k_add_interior<2, T>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, u, e, run);
+      launch_after(k_add_interior<2, T>, split_grid(k_add_interior<2, T>, nchunks), kThreads, 0, s, patches, chunks, nchunks, u, e, run);
    else
-      k_add_interior<3, T><<<split_grid(k_add_interior<3, T>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, u, e, run);
+      launch_after(k_add_interior<3, T>, split_grid(k_add_interior<3, T>, nchunks), kThreads, 0, s, patches, chunks, nchunks, u, e, run);
 }
 
 template <class S, class D>
@@ -2400,7 +2426,7 @@ void launch_convert(cudaStream_t s, const S *src, D *dst, long long n)
 {
    if (n <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
-   k_convert<S, D><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(src, dst, n);
+   launch_after(k_convert<S, D>, (unsigned)((n + 255) / 256), 256, 0, s, src, dst, n);
 }
 
 void launch_reduce(cudaStream_t s, int dim, int mode, const ReduceLevels &lv, int nprob,
@@ -2408,8 +2434,8 @@ void launch_reduce(cudaStream_t s, int dim, int mode, const ReduceLevels &lv, in
 {
    const int n = lv.first[lv.n];
    g_launches.fetch_add(n > 0 ? 2 : 1, std::memory_order_relaxed);
-#define VP(D, M) k_reduce_partial<D, M><<<work_grid(k_reduce_partial<D, M>, n), kThreads, 0, s>>>(lv)
-#define VR(M) k_reduce_levels<M><<<nprob, kThreads, 0, s>>>(lv, acc, host, err, host_err)
+#define VP(D, M) launch_after(k_reduce_partial<D, M>, work_grid(k_reduce_partial<D, M>, n), kThreads, 0, s, lv)
+#define VR(M) launch_after(k_reduce_levels<M>, nprob, kThreads, 0, s, lv, acc, host, err, host_err)
    if (mode == kReduceDot) {
       if (n > 0) {
          if (dim == 2) VP(2, kReduceDot);
@@ -2440,11 +2466,9 @@ void launch_vec_lincomb(cudaStream_t s, int dim, int nchunks, const PatchDesc *p
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
    if (dim == 2)
-      k_vec_lincomb<2><<<split_grid(k_vec_lincomb<2>, nchunks), kThreads, 0, s>>>(
-         patches, chunks, nchunks, z, zg, x, xg, y, yg, a, b);
+      launch_after(k_vec_lincomb<2>, split_grid(k_vec_lincomb<2>, nchunks), kThreads, 0, s, patches, chunks, nchunks, z, zg, x, xg, y, yg, a, b);
    else
-      k_vec_lincomb<3><<<split_grid(k_vec_lincomb<3>, nchunks), kThreads, 0, s>>>(
-         patches, chunks, nchunks, z, zg, x, xg, y, yg, a, b);
+      launch_after(k_vec_lincomb<3>, split_grid(k_vec_lincomb<3>, nchunks), kThreads, 0, s, patches, chunks, nchunks, z, zg, x, xg, y, yg, a, b);
 }
 
 void launch_sweep_check(cudaStream_t s, const unsigned long long *red,
@@ -2453,14 +2477,14 @@ void launch_sweep_check(cudaStream_t s, const unsigned long long *red,
 {
    g_launches.fetch_add(1, std::memory_order_relaxed);
    const int nb = (nprob + 127) / 128;
-   k_sweep_check<<<nb, 128, 0, s>>>(red, blk, last_patch, nprob, tol, run, sweeps);
+   launch_after(k_sweep_check, nb, 128, 0, s, red, blk, last_patch, nprob, tol, run, sweeps);
 }
 
 void launch_accumulate(cudaStream_t s, const long long *src, long long *dst, int n)
 {
    if (n <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
-   k_accumulate<<<(n + 127) / 128, 128, 0, s>>>(src, dst, n);
+   launch_after(k_accumulate, (n + 127) / 128, 128, 0, s, src, dst, n);
 }
 
 void launch_g0_to_g1(cudaStream_t s, int dim, int nchunks, const PatchDesc *patches,
@@ -2468,8 +2492,8 @@ void launch_g0_to_g1(cudaStream_t s, int dim, int nchunks, const PatchDesc *patc
 {
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
-   if (dim == 2) k_g0_to_g1<2><<<split_grid(k_g0_to_g1<2>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, src, dst);
-   else k_g0_to_g1<3><<<split_grid(k_g0_to_g1<3>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, src, dst);
+   if (dim == 2) launch_after(k_g0_to_g1<2>, split_grid(k_g0_to_g1<2>, nchunks), kThreads, 0, s, patches, chunks, nchunks, src, dst);
+   else launch_after(k_g0_to_g1<3>, split_grid(k_g0_to_g1<3>, nchunks), kThreads, 0, s, patches, chunks, nchunks, src, dst);
 }
 
 void launch_patch_rms(cudaStream_t s, int dim, int npatch, const PatchDesc *patches,
@@ -2477,8 +2501,8 @@ void launch_patch_rms(cudaStream_t s, int dim, int npatch, const PatchDesc *patc
 {
    if (npatch <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
-   if (dim == 2) k_patch_rms<2><<<npatch, kThreads, 0, s>>>(patches, x, rms);
-   else k_patch_rms<3><<<npatch, kThreads, 0, s>>>(patches, x, rms);
+   if (dim == 2) launch_after(k_patch_rms<2>, npatch, kThreads, 0, s, patches, x, rms);
+   else launch_after(k_patch_rms<3>, npatch, kThreads, 0, s, patches, x, rms);
 }
 
 void launch_gather_samples(cudaStream_t s, int dim, int npatch, const PatchDesc *patches,
@@ -2488,8 +2512,8 @@ void launch_gather_samples(cudaStream_t s, int dim, int npatch, const PatchDesc 
    g_launches.fetch_add(1, std::memory_order_relaxed);
    const long long S3 = (long long)S * S * S;
    dim3 grid((unsigned)((S3 + kThreads - 1) / kThreads), (unsigned)npatch);
-   if (dim == 2) k_gather_samples<2><<<grid, kThreads, 0, s>>>(patches, x, scale, out, S);
-   else k_gather_samples<3><<<grid, kThreads, 0, s>>>(patches, x, scale, out, S);
+   if (dim == 2) launch_after(k_gather_samples<2>, grid, kThreads, 0, s, patches, x, scale, out, S);
+   else launch_after(k_gather_samples<3>, grid, kThreads, 0, s, patches, x, scale, out, S);
 }
 
 void launch_scatter_samples(cudaStream_t s, int dim, int nchunks, const PatchDesc *patches,
@@ -2499,9 +2523,9 @@ void launch_scatter_samples(cudaStream_t s, int dim, int nchunks, const PatchDes
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
    if (dim == 2)
-      k_scatter_samples<2><<<split_grid(k_scatter_samples<2>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, y, scale, S, dst);
+      launch_after(k_scatter_samples<2>, split_grid(k_scatter_samples<2>, nchunks), kThreads, 0, s, patches, chunks, nchunks, y, scale, S, dst);
    else
-      k_scatter_samples<3><<<split_grid(k_scatter_samples<3>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, y, scale, S, dst);
+      launch_after(k_scatter_samples<3>, split_grid(k_scatter_samples<3>, nchunks), kThreads, 0, s, patches, chunks, nchunks, y, scale, S, dst);
 }
 
 void launch_dot_pair(cudaStream_t s, int dim, int nchunks, const PatchDesc *patches,
@@ -2511,17 +2535,17 @@ void launch_dot_pair(cudaStream_t s, int dim, int nchunks, const PatchDesc *patc
    if (nchunks <= 0) return;
    g_launches.fetch_add(2, std::memory_order_relaxed);
    if (dim == 2)
-      k_dot_pair<2><<<work_grid(k_dot_pair<2>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, r, r2, w, partial);
+      launch_after(k_dot_pair<2>, work_grid(k_dot_pair<2>, nchunks), kThreads, 0, s, patches, chunks, nchunks, r, r2, w, partial);
    else
-      k_dot_pair<3><<<work_grid(k_dot_pair<3>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, r, r2, w, partial);
-   k_norm_reduce<<<nprob, kThreads, 0, s>>>(partial, prob_chunk_begin, nprob, acc);
+      launch_after(k_dot_pair<3>, work_grid(k_dot_pair<3>, nchunks), kThreads, 0, s, patches, chunks, nchunks, r, r2, w, partial);
+   launch_after(k_norm_reduce, nprob, kThreads, 0, s, partial, prob_chunk_begin, nprob, acc);
 }
 
 void launch_alpha(cudaStream_t s, const double2 *acc, const int *active, int nprob,
                   double *alpha)
 {
    g_launches.fetch_add(1, std::memory_order_relaxed);
-   k_alpha<<<(nprob + 127) / 128, 128, 0, s>>>(acc, active, nprob, alpha);
+   launch_after(k_alpha, (nprob + 127) / 128, 128, 0, s, acc, active, nprob, alpha);
 }
 
 void launch_apply_alpha(cudaStream_t s, int dim, int nchunks, const PatchDesc *patches,
@@ -2531,9 +2555,9 @@ void launch_apply_alpha(cudaStream_t s, int dim, int nchunks, const PatchDesc *p
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
    if (dim == 2)
-      k_apply_alpha<2><<<split_grid(k_apply_alpha<2>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, alpha, u, e, r, r2);
+      launch_after(k_apply_alpha<2>, split_grid(k_apply_alpha<2>, nchunks), kThreads, 0, s, patches, chunks, nchunks, alpha, u, e, r, r2);
    else
-      k_apply_alpha<3><<<split_grid(k_apply_alpha<3>, nchunks), kThreads, 0, s>>>(patches, chunks, nchunks, alpha, u, e, r, r2);
+      launch_after(k_apply_alpha<3>, split_grid(k_apply_alpha<3>, nchunks), kThreads, 0, s, patches, chunks, nchunks, alpha, u, e, r, r2);
 }
 
 void launch_gather(cudaStream_t s, const long long *idx, long long n, const double *src,
@@ -2541,7 +2565,7 @@ void launch_gather(cudaStream_t s, const long long *idx, long long n, const doub
 {
    if (n <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
-   k_gather<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(idx, n, src, dst);
+   launch_after(k_gather, (unsigned)((n + 255) / 256), 256, 0, s, idx, n, src, dst);
 }
 
 void launch_scatter(cudaStream_t s, const long long *idx, long long n, const double *src,
@@ -2549,7 +2573,7 @@ void launch_scatter(cudaStream_t s, const long long *idx, long long n, const dou
 {
    if (n <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
-   k_scatter<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(idx, n, src, dst);
+   launch_after(k_scatter, (unsigned)((n + 255) / 256), 256, 0, s, idx, n, src, dst);
 }
 
 // explicit instantiations: FP64 (reference arithmetic) and FP32 (mixed

@@ -28,6 +28,7 @@ k_adaption_tags(const PatchDesc *__restrict__ patches, const Chunk *__restrict__
                 unsigned char *__restrict__ tags, unsigned long long *__restrict__ counts,
                 const int *__restrict__ run)
 {
+   pdl_begin();
    __shared__ unsigned cnt[kThreads / 32];
    WORK_LOOP(ch) {
       const PatchDesc &p = patches[ch.patch];
@@ -89,6 +90,7 @@ k_tags_dense(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ ch
              const unsigned char *__restrict__ tags, int prob, int3 lo, int3 n,
              unsigned char *__restrict__ dense)
 {
+   pdl_begin();
    WORK_LOOP(ch) {
       const PatchDesc &p = patches[ch.patch];
       if (p.prob != prob) continue;
@@ -116,6 +118,7 @@ __global__ void __launch_bounds__(kBrThreads)
 k_br_histogram(const BrItem *__restrict__ items, const BrNode *__restrict__ nodes,
                const unsigned char *__restrict__ dense_all, int *__restrict__ hist)
 {
+   pdl_begin();
    __shared__ int wsum[kBrThreads / 32];
    const BrItem it = items[blockIdx.x];
    const BrNode nd = nodes[it.node];
@@ -170,11 +173,9 @@ void launch_adaption_tags(cudaStream_t s, int dim, int nchunks, const PatchDesc 
    if (nchunks <= 0) return;
    add_kernel_launches(1);
    if (dim == 2)
-      k_adaption_tags<2><<<work_grid(k_adaption_tags<2>, nchunks), kThreads, 0, s>>>(
-         patches, chunks, nchunks, u, threshold, tags, counts, run);
+      launch_after(k_adaption_tags<2>, work_grid(k_adaption_tags<2>, nchunks), kThreads, 0, s, patches, chunks, nchunks, u, threshold, tags, counts, run);
    else
-      k_adaption_tags<3><<<work_grid(k_adaption_tags<3>, nchunks), kThreads, 0, s>>>(
-         patches, chunks, nchunks, u, threshold, tags, counts, run);
+      launch_after(k_adaption_tags<3>, work_grid(k_adaption_tags<3>, nchunks), kThreads, 0, s, patches, chunks, nchunks, u, threshold, tags, counts, run);
 }
 
 void launch_tags_dense(cudaStream_t s, int dim, int nchunks, const PatchDesc *patches,
@@ -185,11 +186,9 @@ void launch_tags_dense(cudaStream_t s, int dim, int nchunks, const PatchDesc *pa
    add_kernel_launches(1);
    const int3 l = make_int3(lo[0], lo[1], lo[2]), e = make_int3(n[0], n[1], n[2]);
    if (dim == 2)
-      k_tags_dense<2><<<work_grid(k_tags_dense<2>, nchunks), kThreads, 0, s>>>(
-         patches, chunks, nchunks, tags, prob, l, e, dense);
+      launch_after(k_tags_dense<2>, work_grid(k_tags_dense<2>, nchunks), kThreads, 0, s, patches, chunks, nchunks, tags, prob, l, e, dense);
    else
-      k_tags_dense<3><<<work_grid(k_tags_dense<3>, nchunks), kThreads, 0, s>>>(
-         patches, chunks, nchunks, tags, prob, l, e, dense);
+      launch_after(k_tags_dense<3>, work_grid(k_tags_dense<3>, nchunks), kThreads, 0, s, patches, chunks, nchunks, tags, prob, l, e, dense);
 }
 
 void launch_br_histogram(cudaStream_t s, int nitems, const BrItem *items, const BrNode *nodes,
@@ -197,7 +196,7 @@ void launch_br_histogram(cudaStream_t s, int nitems, const BrItem *items, const 
 {
    if (nitems <= 0) return;
    add_kernel_launches(1);
-   k_br_histogram<<<nitems, kBrThreads, 0, s>>>(items, nodes, dense, hist);
+   launch_after(k_br_histogram, nitems, kBrThreads, 0, s, items, nodes, dense, hist);
 }
 
 }  // namespace samrai_b200

@@ -502,6 +502,7 @@ k_rb_staged(const Chunk *__restrict__ chunks, int nwork, const UnitCopy *__restr
             StageBases bases, int stage_bytes, int depth, ColourPass<DIM, DVAR, CKIND, T> pass,
             int *__restrict__ err, WaitTest wt)
 {
+   pdl_begin();
    staged_walk(chunks, nwork, copies, bases, stage_bytes, depth, err, wt, pass);
 }
 
@@ -623,6 +624,7 @@ k_res_staged(const Chunk *__restrict__ chunks, int nwork, const UnitCopy *__rest
              StageBases bases, int stage_bytes, int depth, ResidualPass<DIM, DVAR, CKIND, TU> pass,
              int *__restrict__ err, WaitTest wt)
 {
+   pdl_begin();
    staged_walk(chunks, nwork, copies, bases, stage_bytes, depth, err, wt, pass);
 }
 
@@ -658,8 +660,7 @@ void res_staged_inst(cudaStream_t s, int nunits, int stage_bytes, int depth, con
    const int smem = kBarrierBytes + depth * stage_bytes;
    const int grid = staged_grid(k_res_staged<DIM, DVAR, CK, TU>, nunits, smem);
    const ResidualPass<DIM, DVAR, CK, TU> pass{dconst, cconst, res, oflux};
-   k_res_staged<DIM, DVAR, CK, TU><<<grid, kStageBlock, smem, s>>>(
-      units, nunits, copies, bases, stage_bytes, depth, pass, err, wt);
+   launch_after(k_res_staged<DIM, DVAR, CK, TU>, grid, kStageBlock, smem, s, units, nunits, copies, bases, stage_bytes, depth, pass, err, wt);
 }
 
 template <int DIM, bool DVAR, int CK, class T>
@@ -685,8 +686,7 @@ void staged_inst(cudaStream_t s, int nunits, int stage_bytes, int depth, const C
    per_sm = per_sm < 1 ? 1 : per_sm;
    const int grid = nunits < nsm * per_sm ? nunits : nsm * per_sm;
    const ColourPass<DIM, DVAR, CK, T> pass{u, offset, (T)dconst, (T)cconst, bc};
-   k_rb_staged<DIM, DVAR, CK, T><<<grid, kStageBlock, smem, s>>>(
-      units, nunits, copies, bases, stage_bytes, depth, pass, err, wt);
+   launch_after(k_rb_staged<DIM, DVAR, CK, T>, grid, kStageBlock, smem, s, units, nunits, copies, bases, stage_bytes, depth, pass, err, wt);
 }
 
 }  // namespace
