@@ -4409,6 +4409,7 @@ long long cluster_levels(fac_ctx *ctx, int ln, const std::vector<int> &probs,
       for (int a = 0; a < 3; ++a) {
          dlo[q][a] = lo[a];
          dn[q][a] = hi[a] - lo[a] + 1;
+         if (a == 0) dn[q][a] = (dn[q][a] + 15) / 16 * 16;  // rows of whole words
          cells *= dn[q][a];
       }
       doff[q + 1] = doff[q] + ((cells + 255) / 256) * 256;
@@ -4465,15 +4466,14 @@ long long cluster_levels(fac_ctx *ctx, int ln, const std::vector<int> &probs,
             nd.dn[a] = dn[q][a];
             e[a] = t.hi[a] - t.lo[a] + 1;
          }
-         if (e[0] > kBrThreads * kBrMaxXPerThread)
+         if (e[0] > kBrMaxX)
             throw FacError(FAC_ERR_ARG, "clustering box too long along x");
          nd.hoff = hsize;
          nd.doff = doff[q];
          hsize += e[0] + e[1] + e[2];
          nodes.push_back(nd);
-         // runs of rows of at most ~64k cells per block
          const int rows = e[1] * e[2];
-         const int per = std::max(1, 65536 / e[0]);
+         const int per = std::min(std::max(1, kBrItemCells / e[0]), kBrMaxRows);
          for (int r0 = 0; r0 < rows; r0 += per) items.push_back({f, r0, std::min(per, rows - r0), 0});
       }
       put(d_nodes, nodes);

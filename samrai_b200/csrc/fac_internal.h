@@ -395,10 +395,13 @@ struct BrItem {
    int nrows;
    int pad;
 };
-// Block of the histogram kernel and x positions per thread: node boxes up
-// to kBrThreads * kBrMaxXPerThread cells along x.
+// The histogram kernel: threads of a block, the longest node box along x, the
+// rows of an item (a lane counts bytewise: at most 255 of a warp's rows) and
+// the cells it is cut for.
 constexpr int kBrThreads = 256;
-constexpr int kBrMaxXPerThread = 4;
+constexpr int kBrMaxX = 1024;
+constexpr int kBrMaxRows = 255 * (kBrThreads / 32);
+constexpr int kBrItemCells = 16384;
 
 // One bulk copy of a staged unit: nbytes (a multiple of 16) from byte
 // src_off (16-byte aligned) of source array src into the stage at dst_off.

@@ -110,58 +110,86 @@ k_tags_dense(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ ch
 // Tag histograms of Berger-Rigoutsos nodes (makeLocalTagHistogram,
 // mesh/BergerRigoutsosNode.C:1186-1241): per node, the number of tags in
 // each index plane normal to each axis.  One block per work item (a run of
-// rows of one node box; a row runs along x): a thread keeps the count of
-// its x positions over the rows, each row's total goes to the node's y and
-// z counts with one atomic.  Integer atomics: the result does not depend
-// on the order.
+// rows of one node box; a row runs along x).  A row is read in words of four
+// tags (the dense arrays' rows are whole words, so a node's x positions keep
+// their byte in every row); a row of up to 128 tags takes as many lanes as it
+// has words, so a warp reads several short rows at once.  A lane adds its words
+// up bytewise (at most 255 rows), rows' totals are reduced among their lanes;
+// both are gathered in shared memory and added to the node's counts once per
+// block.  Integer atomics: the result does not depend on the order.
+//
+// Bound by the latency of the tag loads, four rows of a lane in flight.  Eight
+// problems of 10.4 million cells, their finest levels: 12.6 us a tree depth on
+// average, 300 with a block of byte loads and two barriers per row; the whole
+// regrid step 7.3 ms and 2.2.
 __global__ void __launch_bounds__(kBrThreads)
 k_br_histogram(const BrItem *__restrict__ items, const BrNode *__restrict__ nodes,
                const unsigned char *__restrict__ dense_all, int *__restrict__ hist)
 {
    pdl_begin();
-   __shared__ int wsum[kBrThreads / 32];
+   __shared__ int xs[kBrMaxX], rows[kBrMaxRows];
    const BrItem it = items[blockIdx.x];
    const BrNode nd = nodes[it.node];
-   const unsigned char *dense = dense_all + nd.doff;
-   const int3 lo = make_int3(nd.dlo[0], nd.dlo[1], nd.dlo[2]);
-   const int3 n = make_int3(nd.dn[0], nd.dn[1], nd.dn[2]);
    const int ex = nd.hi[0] - nd.lo[0] + 1, ey = nd.hi[1] - nd.lo[1] + 1;
    int *hx = hist + nd.hoff, *hy = hx + ex, *hz = hy + ey;
    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-   // x positions of this thread: threadIdx.x + k kBrThreads, k < kBrMaxXPerThread
-   int xc[kBrMaxXPerThread];
+   for (int i = threadIdx.x; i < ex; i += kBrThreads) xs[i] = 0;
+   for (int i = threadIdx.x; i < it.nrows; i += kBrThreads) rows[i] = 0;
+   __syncthreads();
+   const int x0 = nd.lo[0] - nd.dlo[0];
+   const int shift = x0 & 3;                    // tags of the first word before the node
+   const int words = (shift + ex + 3) >> 2;
+   int lanes = 1;                               // per row
+   while (lanes < words && lanes < 32) lanes *= 2;
+   const int wl = lane & (lanes - 1), per = 32 / lanes;
+   const int first = wid * per + lane / lanes, step = kBrThreads / 32 * per;
+   const long long pitch = nd.dn[0], plane = pitch * nd.dn[1];
+   const unsigned char *base = dense_all + nd.doff + (x0 - shift) +
+                               pitch * (nd.lo[1] - nd.dlo[1]) + plane * (nd.lo[2] - nd.dlo[2]);
+   for (int w0 = 0; w0 < words; w0 += lanes) {
+      const int w = w0 + wl;
+      // bytes of this lane's word inside the node
+      unsigned mask = 0;
 #pragma unroll
-   for (int k = 0; k < kBrMaxXPerThread; ++k) xc[k] = 0;
-   for (int r = it.row0; r < it.row0 + it.nrows; ++r) {
-      const int ry = r % ey, rz = r / ey;
-      const long long y = nd.lo[1] + ry - lo.y, z = nd.lo[2] + rz - lo.z;
-      const unsigned char *row = dense + (nd.lo[0] - lo.x) + (long long)n.x * (y + (long long)n.y * z);
-      int rc = 0;
-#pragma unroll
-      for (int k = 0; k < kBrMaxXPerThread; ++k) {
-         const int x = threadIdx.x + k * kBrThreads;
-         const int v = x < ex ? row[x] : 0;
-         xc[k] += v;
-         rc += v;
+      for (int q = 0; q < 4; ++q) {
+         const int x = 4 * w + q - shift;
+         if (x >= 0 && x < ex) mask |= 1u << (8 * q);
       }
-      for (int o = 16; o > 0; o >>= 1) rc += __shfl_down_sync(0xffffffffu, rc, o);
-      if (lane == 0) wsum[wid] = rc;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-         int s = 0;
-         for (int w = 0; w < kBrThreads / 32; ++w) s += wsum[w];
-         if (s) {
-            atomicAdd(hy + ry, s);
-            atomicAdd(hz + rz, s);
+      unsigned sum = 0;  // four counts
+      for (int r0 = 0; r0 < it.nrows; r0 += 4 * step) {
+         unsigned v[4];
+#pragma unroll
+         for (int q = 0; q < 4; ++q) {
+            const int r = r0 + first + q * step, g = it.row0 + r;
+            v[q] = 0;
+            if (r < it.nrows && mask)
+               v[q] = *reinterpret_cast<const unsigned *>(base + 4 * w + pitch * (g % ey) +
+                                                          plane * (g / ey)) & mask;
+         }
+#pragma unroll
+         for (int q = 0; q < 4; ++q) {
+            const int r = r0 + first + q * step;
+            sum += v[q];
+            int c = __popc(v[q]);
+            for (int o = lanes / 2; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+            if (wl == 0 && r < it.nrows && c) rows[r] += c;  // this lane's row alone
          }
       }
-      __syncthreads();
-   }
 #pragma unroll
-   for (int k = 0; k < kBrMaxXPerThread; ++k) {
-      const int x = threadIdx.x + k * kBrThreads;
-      if (x < ex && xc[k]) atomicAdd(hx + x, xc[k]);
+      for (int q = 0; q < 4; ++q) {
+         const int c = (int)((sum >> (8 * q)) & 0xffu);
+         if (c) atomicAdd(&xs[4 * w + q - shift], c);
+      }
    }
+   __syncthreads();
+   for (int i = threadIdx.x; i < ex; i += kBrThreads)
+      if (xs[i]) atomicAdd(hx + i, xs[i]);
+   for (int i = threadIdx.x; i < it.nrows; i += kBrThreads)
+      if (rows[i]) {
+         const int g = it.row0 + i;
+         atomicAdd(hy + g % ey, rows[i]);
+         atomicAdd(hz + g / ey, rows[i]);
+      }
 }
 
 }  // namespace

@@ -93,3 +93,41 @@ def test_cluster_all_problems_at_once(require_gpu):
     fx, _ = _fixture(names[0])
     assert np.array_equal(br_cases.sorted_boxes(allb[0]), br_cases.sorted_boxes(fx["boxes"]))
     g.close()
+
+
+@pytest.mark.parametrize("n, bounds", [
+    # rows of 1 to 1024 tags, bounds whose first cell lies on every byte of a word
+    ((1024, 3), [[0, 0, 1023, 2]]),
+    ((700, 9), [[1, 0, 350, 8], [351, 2, 698, 8]]),
+    ((37, 2100), [[2, 0, 36, 2099]]),
+    ((130, 8, 5), [[3, 1, 0, 127, 7, 4], [128, 0, 0, 129, 7, 4]]),
+    ((5, 70, 40), [[0, 0, 0, 4, 69, 39]]),
+])
+def test_histograms_of_long_and_ragged_rows(n, bounds, require_gpu):
+    """Node boxes at the edges of the histogram kernel's split (words of four
+    tags, lanes per row, rows per block): the boxes of the CPU restatement."""
+    from oracle import br_oracle
+    from samrai_b200 import configs
+    dim = len(n)
+    m = tuple(n) + (1,) * (3 - dim)
+    p = configs.Problem(dim=dim, n0=m, xlo=(0.0,) * 3, xup=(1.0,) * 3,
+                        levels=[configs.Level((1, 1, 1), np.array([[0, 0, 0] + [x - 1 for x in m]],
+                                                                  dtype=np.int32))])
+    rng = np.random.default_rng(sum(m))
+    shape = [x + 2 for x in m[:dim]][::-1]
+    u = np.zeros(shape)
+    for _ in range(12):  # spikes tag their neighbourhoods
+        u[tuple(rng.integers(0, s) for s in shape)] = 1.0
+    ctx = fac.FacContext([p])
+    ctx.upload(U, 0, 0, u.reshape(-1))
+    ctx.tag_gradient(U, 0, 0.4)
+    tags = ctx.download_tags(0, 0).reshape(m[::-1])
+    full = [b if dim == 3 else [b[0], b[1], 0, b[2], b[3], 0] for b in bounds]
+    got = ctx.cluster_tags(0, 0, full, [2] * dim)
+    cl = br_oracle.Clusterer(tags if dim == 3 else tags[0], [0, 0, 0], dim, [2] * dim, None, 0.8, 0.8)
+    boxes = cl.cluster(full)
+    pad = [0] * (3 - dim)
+    want = np.array([list(lo) + pad + list(hi) + pad for lo, hi in boxes], dtype=np.int64)
+    assert len(want) > 0
+    assert np.array_equal(br_cases.sorted_boxes(got), br_cases.sorted_boxes(want))
+    ctx.close()
