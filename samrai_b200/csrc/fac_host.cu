@@ -290,7 +290,8 @@ struct HostProblem {
    std::vector<Box> boxes[kMaxLevels];
 };
 
-// internal field id: the all-zero ghost-0 field
+// internal field id: no right-hand side (the operator application A x), null to
+// the kernels
 constexpr int kFieldZero = 100;
 
 struct LevelState {
@@ -309,7 +310,6 @@ struct LevelState {
 
    DevArray<PatchDesc> d_patches;
    DevArray<double> u, e, f, r, tr, w, c, d, flux, oflux, cfflux;
-   DevArray<double> zero;  // all-zero ghost-0 field (right-hand side of A x)
    // Krylov workspace (fac_solve_fgmres): V_0..V_m then Z_0..Z_{m-1}, n0
    // apart, and per-chunk partial sums of the multi-dot products
    DevArray<double> kry, kry_partial;
@@ -345,6 +345,7 @@ struct LevelState {
    // cells the staged residual leaves to the fix-up pass
    std::vector<CellRef> rfix;
    DevArray<CellRef> d_rfix;
+   int rfix_open = 0;  // the first of them: the uncovered cells
    // host copies of cfmask and fcmask
    std::vector<unsigned char> cfmask_h, fcmask_h;
    // regrid step: tags of the level's cells (ghost-0 layout), allocated on first use
@@ -376,6 +377,9 @@ struct LevelState {
    DevArray<CfFace> d_cf;
    ItemList<RestrictItem> restrict_g1, restrict_g0;  // from level ln+1 into this
    ItemList<FluxCoarsenItem> fcoarsen;               // from level ln+1 into this
+   ItemList<FluxCoarsenItem> fcoarsen_open;          // those of faces of uncovered cells
+   std::vector<unsigned char> cov;                   // ghost-0 cells under the finer level,
+                                                     // while the tables are built
    ItemList<FillItem> tmp_fill;                      // coarse interpolation arrays
    ItemList<ProlongItem> prolong;                    // from level ln-1 into this
    ItemList<ProlongItem> prolong2;                   // the same, counted in coarse cells
@@ -481,6 +485,7 @@ struct fac_ctx {
    // derived again from the caller's level 0 before the next solve
    int ext_levels = 0;
    bool ext_dirty = false;
+   int low = 0;  // leading levels that are covered throughout (first_level)
    // learned correction after every cycle (fac_set_learned)
    fac_cnn *cnn = nullptr;
    int learned_level = -1;
@@ -673,7 +678,7 @@ void harvest_graph_profile(fac_ctx *c)
 double *field_ptr(LevelState &L, int fid)
 {
    switch (fid) {
-      case kFieldZero: return L.zero.p;
+      case kFieldZero: return nullptr;
       case FAC_U: return L.u.p;
       case FAC_F: return L.f.p;
       case FAC_E: return L.e.p;
@@ -1383,6 +1388,12 @@ void build_residual_fixups(fac_ctx *c, int ln)
       for (size_t q = 0; q < mark.size(); ++q)
          if (mark[q]) L.rfix.push_back({ip, (int)q});
    }
+   // the uncovered cells first: a residual that is restricted from the finer
+   // level next (residual_open) takes no others
+   const auto open = std::stable_partition(L.rfix.begin(), L.rfix.end(), [&](const CellRef &r) {
+      return !L.cov[L.hp[r.patch].off0 + r.lin];
+   });
+   L.rfix_open = (int)(open - L.rfix.begin());
    L.d_rfix.upload(L.rfix, c->stream);
 }
 
@@ -1850,6 +1861,36 @@ void build_chunks(fac_ctx *c, int ln)
 }
 
 // Inter-level tables with the next finer level (restriction, flux coarsening).
+// The cells of a level that lie under the next finer one.
+void build_covered(fac_ctx *c, int ln)
+{
+   LevelState &L = c->L[ln];
+   L.cov.assign((size_t)std::max<long long>(1, L.n0), 0);
+   L.covered = false;
+   if (ln + 1 >= c->nlev) return;
+   const LevelState &Fl = c->L[ln + 1];
+   long long n = 0;
+   for (int ip = 0; ip < L.npatch; ++ip) {
+      const Box &b = L.box[ip];
+      const int p = L.hp[ip].prob;
+      const long long nx = b.hi[0] - b.lo[0] + 1, ny = b.hi[1] - b.lo[1] + 1;
+      for (int iq = Fl.prob_patch_begin[p]; iq < Fl.prob_patch_begin[p + 1]; ++iq) {
+         const Box ov = isect(coarsen(Fl.box[iq], c->dim, Fl.ratio), b);
+         if (ov.empty()) continue;
+         for (int k = ov.lo[2]; k <= ov.hi[2]; ++k)
+            for (int j = ov.lo[1]; j <= ov.hi[1]; ++j) {
+               unsigned char *row =
+                  &L.cov[L.hp[ip].off0 + nx * ((j - b.lo[1]) + ny * (k - b.lo[2])) - b.lo[0]];
+               for (int i = ov.lo[0]; i <= ov.hi[0]; ++i) {
+                  n += row[i] == 0;
+                  row[i] = 1;
+               }
+            }
+      }
+   }
+   L.covered = L.n0 > 0 && n == L.n0;
+}
+
 void build_coarsen_tables(fac_ctx *c, int ln)
 {
    LevelState &C = c->L[ln];
@@ -1859,6 +1900,7 @@ void build_coarsen_tables(fac_ctx *c, int ln)
    C.restrict_g1.clear();
    C.restrict_g0.clear();
    C.fcoarsen.clear();
+   C.fcoarsen_open.clear();
    const int *r = Fl.ratio;
    const int raux = r[0] | (r[1] << 8) | ((dim == 3 ? r[2] : 1) << 16);
    for (int p = 0; p < np; ++p) {
@@ -1952,12 +1994,28 @@ void build_coarsen_tables(fac_ctx *c, int ln)
                piece.hi[d] = k.hi[d];
             }
             C.fcoarsen.add(piece, k.size());
+            // a face matters to an uncovered cell of its patch on either side
+            const PatchDesc &cp = C.hp[piece.coarse_patch];
+            const long long nx = cp.hi[0] - cp.lo[0] + 1, ny = cp.hi[1] - cp.lo[1] + 1;
+            bool open = false;
+            for (int z = k.lo[2]; z <= k.hi[2] && !open; ++z)
+               for (int y = k.lo[1]; y <= k.hi[1] && !open; ++y)
+                  for (int x = k.lo[0]; x <= k.hi[0] && !open; ++x)
+                     for (int sd = 0; sd < 2; ++sd) {
+                        int q[3] = {x, y, z};
+                        q[it.axis] -= sd;
+                        if (q[it.axis] < cp.lo[it.axis] || q[it.axis] > cp.hi[it.axis]) continue;
+                        open = open || !C.cov[cp.off0 + (q[0] - cp.lo[0]) +
+                                              nx * ((q[1] - cp.lo[1]) + ny * (q[2] - cp.lo[2]))];
+                     }
+            if (open) C.fcoarsen_open.add(piece, k.size());
          }
       }
    }
    C.restrict_g1.upload(c->stream);
    C.restrict_g0.upload(c->stream);
    C.fcoarsen.upload(c->stream);
+   C.fcoarsen_open.upload(c->stream);
    // faces of level ln written by the flux coarsening
    std::vector<unsigned char> fm(std::max<long long>(1, C.ns), 0);
    for (const FluxCoarsenItem &it : C.fcoarsen.items) {
@@ -2118,32 +2176,19 @@ void compute_weights_host(fac_ctx *c)
    const int dim = c->dim;
    for (int ln = c->nlev - 1; ln >= 0; --ln) {
       LevelState &L = c->L[ln];
+      if (L.cov.empty()) build_covered(c, ln);
       std::vector<double> w(std::max<long long>(1, L.n0), 0.0);
       for (int ip = 0; ip < L.npatch; ++ip) {
          const int p = L.hp[ip].prob;
          double vol = L.dx[3 * p + 0];
          vol *= L.dx[3 * p + 1];
          if (dim > 2) vol *= L.dx[3 * p + 2];
-         const Box &b = L.box[ip];
-         const long long n = b.size();
-         for (long long t = 0; t < n; ++t) w[L.hp[ip].off0 + t] = vol;
-         if (ln < c->nlev - 1) {
-            LevelState &Fl = c->L[ln + 1];
-            const long long nx = b.hi[0] - b.lo[0] + 1, ny = b.hi[1] - b.lo[1] + 1;
-            for (int iq = Fl.prob_patch_begin[p]; iq < Fl.prob_patch_begin[p + 1]; ++iq) {
-               Box ov = isect(coarsen(Fl.box[iq], dim, Fl.ratio), b);
-               if (ov.empty()) continue;
-               for (int k = ov.lo[2]; k <= ov.hi[2]; ++k)
-                  for (int j = ov.lo[1]; j <= ov.hi[1]; ++j)
-                     for (int i = ov.lo[0]; i <= ov.hi[0]; ++i)
-                        w[L.hp[ip].off0 + (i - b.lo[0]) + nx * ((j - b.lo[1]) + ny * (k - b.lo[2]))] =
-                           0.0;
-            }
-         }
+         const long long o = L.hp[ip].off0, n = L.box[ip].size();
+         for (long long t = o; t < o + n; ++t) w[t] = L.cov[t] ? 0.0 : vol;
       }
-      L.covered = L.n0 > 0 && std::all_of(w.begin(), w.end(), [](double v) { return v == 0.0; });
       CUDA_CHECK(cudaMemcpyAsync(L.w.p, w.data(), L.n0 * sizeof(double), cudaMemcpyHostToDevice,
                                  c->stream));
+      std::vector<unsigned char>().swap(L.cov);
    }
 }
 
@@ -2360,6 +2405,7 @@ void validate_tables(fac_ctx *c)
       validate_chunks(L.restrict_g1, "restrict chunk range");
       validate_chunks(L.restrict_g0, "restrict chunk range");
       validate_chunks(L.fcoarsen, "flux coarsening chunk range");
+      validate_chunks(L.fcoarsen_open, "flux coarsening chunk range");
       validate_chunks(L.tmp_fill, "coarse interpolation chunk range");
       validate_chunks(L.prolong, "prolongation chunk range");
    }
@@ -2413,6 +2459,7 @@ void register_work_lists(fac_ctx *c)
       register_items(c, L.restrict_g1);
       register_items(c, L.restrict_g0);
       register_items(c, L.fcoarsen);
+      register_items(c, L.fcoarsen_open);
       register_items(c, L.tmp_fill);
       if (L.gather_tmp.ok) register_items(c, L.gather_tmp.bc);
       register_items(c, L.prolong);
@@ -2469,8 +2516,6 @@ void initialize(fac_ctx *c)
       L.flux.alloc(std::max<long long>(1, L.ns));
       L.oflux.alloc(std::max<long long>(1, L.no));
       L.cfflux.alloc(std::max<long long>(1, L.no));
-      L.zero.alloc(n0);
-      if (!g_dry) CUDA_CHECK(cudaMemsetAsync(L.zero.p, 0, n0 * sizeof(double), c->stream));
       if (!g_dry)
          for (auto *b : {&L.u, &L.e, &L.f, &L.r, &L.tr, &L.w, &L.c, &L.d, &L.flux, &L.oflux,
                          &L.cfflux})
@@ -2496,6 +2541,9 @@ void initialize(fac_ctx *c)
       build_dirichlet_index(c, ln);
       if (ln > 0) build_prolong_tables(c, ln);
    }
+   for (int ln = 0; ln < c->nlev; ++ln) build_covered(c, ln);
+   c->low = 0;
+   while (c->low < c->nlev && c->L[c->low].covered) ++c->low;
    for (int ln = 0; ln + 1 < c->nlev; ++ln) build_coarsen_tables(c, ln);
    for (int ln = 0; ln < c->nlev; ++ln) {
       build_res_units(c, ln);
@@ -2562,17 +2610,24 @@ void smooth(fac_ctx *c, int fid_e, int fid_r, int ln, int nsweeps, double tol)
    const int np = nprob(c);
    double *e = field_ptr(L, fid_e);
    const double *r = field_ptr(L, fid_r);
-   CUDA_CHECK(cudaMemcpyAsync(c->run.p, c->active.p, np * sizeof(int), cudaMemcpyDeviceToDevice,
-                              c->stream));
-   CUDA_CHECK(cudaMemsetAsync(c->sweeps_call.p, 0, np * sizeof(long long), c->stream));
+   // A fixed sweep count needs no flags of its own, no residual maxima and no
+   // checks, each a launch or a memset: the active problems take them all.
+   // The counts on the device are those of the coarsest level's solves.
+   const bool fixed = tol < 0.0;
+   const int *run = fixed ? c->active.p : c->run.p;
+   if (!fixed)
+      CUDA_CHECK(cudaMemcpyAsync(c->run.p, c->active.p, np * sizeof(int), cudaMemcpyDeviceToDevice,
+                                 c->stream));
+   if (!fixed || ln == 0)
+      CUDA_CHECK(cudaMemsetAsync(c->sweeps_call.p, 0, np * sizeof(long long), c->stream));
    const long long *fmap = (c->fused && L.fused_ok && !c->bc_faces) ? L.facemap.p : nullptr;
    // the staged pass computes no residual maxima: fixed sweep counts only
    const bool staged = fmap && c->staged && tol < 0.0 && L.unit_smem[0] > 0;
    // The fill with the coarser level is a full fill.  Pulling fused passes
    // read only its coarse-fine ghosts; staged passes read face ghost cells,
    // which their pushes keep current after this fill.
-   if (ln > 0) ghost_fill(c, fid_e, ln, true, 1, c->run.p);
-   else if (!fmap || staged) ghost_fill(c, fid_e, ln, false, 1, c->run.p);
+   if (ln > 0) ghost_fill(c, fid_e, ln, true, 1, run);
+   else if (!fmap || staged) ghost_fill(c, fid_e, ln, false, 1, run);
    std::vector<int> hrun(np);
    // smoothing to a tolerance on the coarsest level: every sweep in one launch
    const bool one_launch = tol >= 0.0 && ln == 0 && fmap && L.coarse_ncta > 0;
@@ -2598,16 +2653,18 @@ void smooth(fac_ctx *c, int fid_e, int fid_r, int ln, int nsweeps, double tol)
          for (int v : hrun) any = any || v;
          if (!any) break;
       }
-      CUDA_CHECK(cudaMemsetAsync(L.maxres_red.p, 0, L.maxres_red.n * sizeof(unsigned long long),
-                                 c->stream));
-      CUDA_CHECK(cudaMemsetAsync(L.maxres_blk.p, 0, L.maxres_blk.n * sizeof(unsigned long long),
-                                 c->stream));
+      if (!fixed) {
+         CUDA_CHECK(cudaMemsetAsync(L.maxres_red.p, 0, L.maxres_red.n * sizeof(unsigned long long),
+                                    c->stream));
+         CUDA_CHECK(cudaMemsetAsync(L.maxres_blk.p, 0, L.maxres_blk.n * sizeof(unsigned long long),
+                                    c->stream));
+      }
       for (int color = 0; color < 2; ++color) {
-         if (!fmap) ghost_fill(c, fid_e, ln, false, 1, c->run.p);
+         if (!fmap) ghost_fill(c, fid_e, ln, false, 1, run);
          if (ln > 0)
             launch_cf_flux(c->stream, L.d_cf.p, (int)L.cf.size(), L.d_patches.p, e, L.d.p,
                            c->spec.d_variable, c->spec.d_const, L.tranwt, L.longwt, L.cfflux.p,
-                           c->run.p);
+                           run);
          const int pi = prof_begin(c, 0, L.rb_bytes_prob, 1.0);
          if (staged)
             launch_rb_staged<double>(c->stream, c->dim, c->spec, (int)L.units[0].size(),
@@ -2618,13 +2675,18 @@ void smooth(fac_ctx *c, int fid_e, int fid_r, int ln, int nsweeps, double tol)
          else
             launch_rbgs(c->stream, c->dim, c->spec, (int)L.slot_chunks.size(), L.d_patches.p,
                         L.d_slot_chunks.p, e, r, L.d.p, L.c.p, L.cfflux.p, L.cfmask.p, color,
-                        color == 0 ? L.maxres_red.p : L.maxres_blk.p, c->run.p, fmap, c->bc);
+                        fixed ? nullptr : (color == 0 ? L.maxres_red.p : L.maxres_blk.p), run, fmap,
+                        c->bc);
          prof_end(c, pi);
       }
-      if (!fmap) ghost_fill(c, fid_e, ln, false, 1, c->run.p);
-      launch_sweep_check(c->stream, L.maxres_red.p, L.maxres_blk.p, L.last_patch.p, np, tol,
-                         c->run.p, c->sweeps_call.p);
+      if (!fmap) ghost_fill(c, fid_e, ln, false, 1, run);
+      if (!fixed)
+         launch_sweep_check(c->stream, L.maxres_red.p, L.maxres_blk.p, L.last_patch.p, np, tol,
+                            c->run.p, c->sweeps_call.p, 1);
    }
+   if (fixed && ln == 0 && nsweeps > 0)
+      launch_sweep_check(c->stream, nullptr, nullptr, nullptr, np, tol, c->active.p,
+                         c->sweeps_call.p, nsweeps);
    // Fused passes leave the same-level ghosts stale; one fill of every active
    // problem gives the ghost values the per-sweep fills would have left (a
    // fill depends only on the interior, which a stopped problem no longer
@@ -2659,7 +2721,11 @@ bool staged_residual_on(const fac_ctx *c, int ln, int kind)
           kStageSmemMax;
 }
 
-void comp_residual(fac_ctx *c, int fid_r, int fid_u, int fid_f, int ln, int error_eq)
+// open: only the values of uncovered cells are wanted (the caller restricts the
+// finer level's residual onto the others next), so fluxes under the finer
+// level and the fix-up of covered cells are left out.
+void comp_residual(fac_ctx *c, int fid_r, int fid_u, int fid_f, int ln, int error_eq,
+                   bool open = false)
 {
    OpTimer ot(c, "comp_residual", ln);
    LevelState &L = c->L[ln];
@@ -2681,9 +2747,9 @@ void comp_residual(fac_ctx *c, int fid_r, int fid_u, int fid_f, int ln, int erro
    }
    if (finer) {
       LevelState &Fl = c->L[ln + 1];
-      launch_flux_coarsen(c->stream, L.fcoarsen.d_items.p, L.fcoarsen.d_chunks.p,
-                          L.fcoarsen.nchunks(), L.fcoarsen.d_prefix.p, Fl.d_patches.p, L.d_patches.p, Fl.oflux.p,
-                          L.flux.p, run);
+      const ItemList<FluxCoarsenItem> &fc = open ? L.fcoarsen_open : L.fcoarsen;
+      launch_flux_coarsen(c->stream, fc.d_items.p, fc.d_chunks.p, fc.nchunks(), fc.d_prefix.p,
+                          Fl.d_patches.p, L.d_patches.p, Fl.oflux.p, L.flux.p, run);
    }
    if (staged) {
       launch_res_staged<double>(c->stream, c->dim, c->spec, (int)L.runits[kind].size(),
@@ -2691,7 +2757,8 @@ void comp_residual(fac_ctx *c, int fid_r, int fid_u, int fid_f, int ln, int erro
                                 L.d_rcopies[kind].p, L.d_rhdrs[kind].p, u,
                                 field_ptr(L, fid_f), L.d.p, L.c.p, field_ptr(L, fid_r),
                                 ln > 0 ? L.oflux.p : nullptr, c->kerr.p, c->wait_test);
-      launch_residual_cells<double>(c->stream, c->dim, c->spec, (int)L.rfix.size(), L.d_rfix.p,
+      launch_residual_cells<double>(c->stream, c->dim, c->spec,
+                                    open ? L.rfix_open : (int)L.rfix.size(), L.d_rfix.p,
                                     L.d_patches.p, u, L.d.p, L.cfmask.p, L.tranwt, L.longwt,
                                     L.d_ratio.p, finer ? L.fcmask.p : nullptr, L.flux.p,
                                     field_ptr(L, fid_f), L.c.p, field_ptr(L, fid_r),
@@ -2836,14 +2903,35 @@ void fac_cycle_recursive(fac_ctx *c, int ln)
    }
 }
 
+// The first level the composite problem lives on.  The levels before it (a
+// coarse extension's) are covered throughout: u, the operator and the residual
+// there are restrictions of the finer level's, which a solve needs at its end
+// only (finish_low_levels) -- their weights are 0, they lend no ghost values,
+// and the cycle sets their right-hand sides and errors itself.
+int first_level(const fac_ctx *c)
+{
+   return c->cnn && c->learned_level < c->low ? 0 : c->low;
+}
+
+// u and the residual on those levels, as every cycle's restrictions would have
+// left them.
+void finish_low_levels(fac_ctx *c)
+{
+   for (int ln = first_level(c) - 1; ln >= 0; --ln) {
+      restrict_solution(c, FAC_U, ln);
+      restrict_op(c, FAC_R, FAC_R, ln);
+   }
+}
+
 // FACPreconditioner::computeFullCompositeResidual (FACPreconditioner.C:775-814).
+// Restricts u on its way down, so a solve does not do so before it.
 void full_composite_residual_launch(fac_ctx *c)
 {
    const int lmax = c->nlev - 1;
    comp_residual(c, FAC_R, FAC_U, FAC_F, lmax, 0);
-   for (int ln = lmax - 1; ln >= 0; --ln) {
+   for (int ln = lmax - 1; ln >= first_level(c); --ln) {
       restrict_solution(c, FAC_U, ln);
-      comp_residual(c, FAC_R, FAC_U, FAC_F, ln, 0);
+      comp_residual(c, FAC_R, FAC_U, FAC_F, ln, 0, true);
       restrict_op(c, FAC_R, FAC_R, ln);
    }
    rms_norm_launch(c, FAC_R);
@@ -3176,7 +3264,7 @@ void solve(fac_ctx *c, int *converged, int *iterations, double *residual)
          zero_field(c, FAC_E);
          fac_cycle_recursive(c, c->nlev - 1);
       }
-      for (int ln = 0; ln < c->nlev; ++ln) {
+      for (int ln = first_level(c); ln < c->nlev; ++ln) {
          LevelState &L = c->L[ln];
          if (c->mixed)
             launch_add_interior<float>(c->stream, c->dim, (int)L.cell_chunks.size(),
@@ -3187,7 +3275,6 @@ void solve(fac_ctx *c, int *converged, int *iterations, double *residual)
                                         L.d_patches.p, L.d_cell_chunks.p, L.u.p, L.e.p,
                                         c->active.p);
       }
-      for (int ln = c->nlev - 2; ln >= 0; --ln) restrict_solution(c, FAC_U, ln);
       full_composite_residual_launch(c);
       if (c->cnn) {
          learned_step(c);
@@ -3254,6 +3341,7 @@ void solve(fac_ctx *c, int *converged, int *iterations, double *residual)
    }
    c->host_active.assign(np, 1);
    set_active(c, c->host_active);
+   finish_low_levels(c);
    dirichlet(c, true);
    CUDA_CHECK(cudaStreamSynchronize(c->stream));
    for (int p = 0; p < np; ++p) {
@@ -3583,11 +3671,11 @@ void fgmres_solve(fac_ctx *c, int m, int *converged, int *iterations, double *re
       // then the composite residual level by level.  Each residual fills
       // its level's ghost cells itself (homogeneous boundary values of the
       // error equation), so the restrictions need no fills of their own.
-      const int lmax = c->nlev - 1;
-      for (int ln = lmax - 1; ln >= 0; --ln) restrict_op(c, FAC_E, FAC_E, ln);
+      const int lmax = c->nlev - 1, low = first_level(c);
+      for (int ln = lmax - 1; ln >= low; --ln) restrict_op(c, FAC_E, FAC_E, ln);
       comp_residual(c, FAC_TR, FAC_E, kFieldZero, lmax, 1);
-      for (int ln = lmax - 1; ln >= 0; --ln) {
-         comp_residual(c, FAC_TR, FAC_E, kFieldZero, ln, 1);
+      for (int ln = lmax - 1; ln >= low; --ln) {
+         comp_residual(c, FAC_TR, FAC_E, kFieldZero, ln, 1, true);
          restrict_op(c, FAC_TR, FAC_TR, ln);
       }
    };
@@ -3805,13 +3893,12 @@ void fgmres_solve(fac_ctx *c, int m, int *converged, int *iterations, double *re
       if (kmax > 0)
          CUDA_CHECK(cudaMemcpyAsync(c->kry_coef.p, yk.data(), (size_t)np * kmax * sizeof(double),
                                     cudaMemcpyHostToDevice, c->stream));
-      for (int ln = 0; ln < c->nlev; ++ln) {
+      for (int ln = first_level(c); ln < c->nlev; ++ln) {
          LevelState &L = c->L[ln];
          launch_add_combination(c->stream, c->dim, (int)L.cell_chunks.size(), L.d_patches.p,
                                 L.d_cell_chunks.p, L.u.p, kry_vec(c, ln, zslot0),
                                 std::max<long long>(1, L.n0), kmax, c->kry_coef.p);
       }
-      for (int ln = c->nlev - 2; ln >= 0; --ln) restrict_solution(c, FAC_U, ln);
       std::vector<double> nr;
       full_composite_residual(c, nr);
       for (int p = 0; p < np; ++p) {
@@ -3823,6 +3910,7 @@ void fgmres_solve(fac_ctx *c, int m, int *converged, int *iterations, double *re
    }
    c->host_active.assign(np, 1);
    set_active(c, c->host_active);
+   finish_low_levels(c);
    dirichlet(c, true);
    CUDA_CHECK(cudaStreamSynchronize(c->stream));
    for (int p = 0; p < np; ++p) {
@@ -5186,7 +5274,12 @@ int fac_smooth(fac_ctx *ctx, int fid_e, int fid_r, int ln, int nsweeps, double t
       if (field_ghost(fid_e) != 1 || field_ghost(fid_r) != 0)
          throw FacError(FAC_ERR_ARG, "smooth needs a ghosted unknown and a ghost-0 rhs");
       smooth(ctx, fid_e, fid_r, ln, nsweeps, tol);
-      if (sweeps) {
+      if (sweeps && tol < 0.0) {
+         // a fixed count: every active problem takes it
+         for (int p = 0; p < nprob(ctx); ++p)
+            sweeps[p] = p >= (int)ctx->host_active.size() || ctx->host_active[p]
+                           ? std::max(0, nsweeps) : 0;
+      } else if (sweeps) {
          std::vector<long long> s(nprob(ctx));
          CUDA_CHECK(cudaMemcpyAsync(s.data(), ctx->sweeps_call.p, s.size() * sizeof(long long),
                                     cudaMemcpyDeviceToHost, ctx->stream));

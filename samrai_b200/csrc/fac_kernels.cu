@@ -586,14 +586,15 @@ k_residual(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ chun
          const double uc =
             (double)u[p.off1 + (li + 1) + gx * (lj + 1) + (DIM == 3 ? gxy * (lk + 1) : 0)];
          const double sf = CKIND == 2 ? cfield[c0] : (CKIND == 1 ? cconst : 0.0);
+         const double fv = f ? f[c0] : 0.0;  // null: the operator's zero right-hand side
          double rv, fzl = 0.0, fzh = 0.0;
          if (DIM == 2) {
-            rv = f[c0] - (dxi * (fxh - fxl) + dyi * (fyh - fyl)) - sf * uc;
+            rv = fv - (dxi * (fxh - fxl) + dyi * (fyh - fyl)) - sf * uc;
          } else {
             const int sz = li + nx * (lj + ny * lk);
             fzl = fz[sz];
             fzh = fz[sz + nx * ny];
-            rv = f[c0] - (dxi * (fxh - fxl) + dyi * (fyh - fyl) + dzi * (fzh - fzl)) - sf * uc;
+            rv = fv - (dxi * (fxh - fxl) + dyi * (fyh - fyl) + dzi * (fzh - fzl)) - sf * uc;
          }
          res[c0] = rv;
          if (oflux) {
@@ -694,11 +695,12 @@ __device__ __forceinline__ void residual_cell(
    }
    const long long c0 = p.off0 + lin;
    const double sf = CKIND == 2 ? cfield[c0] : (CKIND == 1 ? cconst : 0.0);
+   const double fv = f ? f[c0] : 0.0;  // null: the operator's zero right-hand side
    double rv;
    if (DIM == 2)
-      rv = f[c0] - (dai[0] * (fl[0][1] - fl[0][0]) + dai[1] * (fl[1][1] - fl[1][0])) - sf * uc;
+      rv = fv - (dai[0] * (fl[0][1] - fl[0][0]) + dai[1] * (fl[1][1] - fl[1][0])) - sf * uc;
    else
-      rv = f[c0] - (dai[0] * (fl[0][1] - fl[0][0]) + dai[1] * (fl[1][1] - fl[1][0]) +
+      rv = fv - (dai[0] * (fl[0][1] - fl[0][0]) + dai[1] * (fl[1][1] - fl[1][0]) +
                     dai[2] * (fl[2][1] - fl[2][0])) -
            sf * uc;
    res[c0] = rv;
@@ -1321,13 +1323,13 @@ __global__ void k_sweep_check(const unsigned long long *__restrict__ red,
                               const unsigned long long *__restrict__ blk,
                               const int *__restrict__ last_patch, int nprob,
                               double tol, int *__restrict__ run,
-                              long long *__restrict__ sweeps)
+                              long long *__restrict__ sweeps, int taken)
 {
    pdl_begin();
    const int pr = blockIdx.x * blockDim.x + threadIdx.x;
    if (pr >= nprob) return;
    if (!run[pr]) return;
-   sweeps[pr] += 1;
+   sweeps[pr] += taken;
    if (tol >= 0.0) {
       const int lp = last_patch[pr];
       const double r = __longlong_as_double((long long)red[lp]);
@@ -2473,11 +2475,11 @@ void launch_vec_lincomb(cudaStream_t s, int dim, int nchunks, const PatchDesc *p
 
 void launch_sweep_check(cudaStream_t s, const unsigned long long *red,
                         const unsigned long long *blk, const int *last_patch, int nprob,
-                        double tol, int *run, long long *sweeps)
+                        double tol, int *run, long long *sweeps, int taken)
 {
    g_launches.fetch_add(1, std::memory_order_relaxed);
    const int nb = (nprob + 127) / 128;
-   launch_after(k_sweep_check, nb, 128, 0, s, red, blk, last_patch, nprob, tol, run, sweeps);
+   launch_after(k_sweep_check, nb, 128, 0, s, red, blk, last_patch, nprob, tol, run, sweeps, taken);
 }
 
 void launch_accumulate(cudaStream_t s, const long long *src, long long *dst, int n)

@@ -222,7 +222,7 @@ void launch_vec_lincomb(cudaStream_t s, int dim, int nchunks, const PatchDesc *p
 
 void launch_sweep_check(cudaStream_t s, const unsigned long long *red,
                         const unsigned long long *blk, const int *last_patch, int nprob,
-                        double tol, int *run, long long *sweeps);
+                        double tol, int *run, long long *sweeps, int taken);
 
 void launch_accumulate(cudaStream_t s, const long long *src, long long *dst, int n);
 
