@@ -441,6 +441,8 @@ int fac_time_interpolate(int dim, const fac_time_box *boxes, int nboxes,
  * FAC_ERR_CUDA; every copy a block issued lands before the block exits, so
  * the context stays usable.  never = 1 makes that wait be for a phase no
  * copy completes: a test of the bound that ends with the error.
+ * The coarsest solve's wait for the values of its cluster's other blocks has
+ * the default limit and reports the same way.
  * fac_clear_device_error resets the flag. */
 int fac_set_wait_test(fac_ctx *ctx, long long limit_cycles, int never);
 int fac_clear_device_error(fac_ctx *ctx);

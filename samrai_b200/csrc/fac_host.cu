@@ -2852,8 +2852,8 @@ void rms_norm_read(fac_ctx *c, std::vector<double> &out)
    const int np = nprob(c);
    CUDA_CHECK(cudaStreamSynchronize(c->stream));
    if (*c->back.err)
-      throw FacError(FAC_ERR_CUDA, "a bounded wait of a staged colour pass ran out (device error "
-                                   "flag; fac_clear_device_error resets it)");
+      throw FacError(FAC_ERR_CUDA, "a bounded wait of a staged colour pass or of the coarsest solve "
+                                   "ran out (device error flag; fac_clear_device_error resets it)");
    const double2 *acc = c->back.acc;
    out.resize(np);
    for (int p = 0; p < np; ++p) {
