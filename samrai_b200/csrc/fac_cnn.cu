@@ -269,14 +269,8 @@ k_conv_mid_tc(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restri
    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
    for (int i = tid; i < kTcShifts * N * 2; i += kTcThreads)
       reinterpret_cast<uint4 *>(ws)[i] = reinterpret_cast<const uint4 *>(wt)[i];
-   // zeros before and after the box of each plane (its positions, halo among
-   // them, are written by every slab's copies)
-   constexpr int kGuard = kTcSpan - kTcBox;
-   for (int i = tid; i < 4 * kGuard; i += kTcThreads) {
-      const int pl = i / kGuard, r = i - pl * kGuard;
-      reinterpret_cast<uint4 *>(tsm)[pl * kTcSpan + (r < kTcFront ? r : r + kTcBox)] =
-         make_uint4(0u, 0u, 0u, 0u);
-   }
+   for (int i = tid; i < 4 * kTcSpan; i += kTcThreads)
+      reinterpret_cast<uint4 *>(tsm)[i] = make_uint4(0u, 0u, 0u, 0u);
    box_cells(tab, tid, kTcThreads);
    if (tid == 0) {
       for (int i = 0; i < 2; ++i)
@@ -774,12 +768,8 @@ k_bwd_weight_mid(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__res
    extern __shared__ __align__(128) unsigned char wsm[];
    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
    constexpr int kFirst = 2 * kTcPlaneBytes, kCells = 16 * kSlabSteps;
-   // zeros around the boxes and in the gradient's cells past the slab
-   for (int i = tid; i < (kFirst + 2 * kCells * 16) / 16; i += kWgThreads) {
-      const int r = i < 2 * kTcSpan ? i % kTcSpan - kTcFront : (i - 2 * kTcSpan) % kCells;
-      if (i < 2 * kTcSpan ? r >= 0 && r < kTcBox : r < kSlabCells) continue;
+   for (int i = tid; i < (kFirst + 2 * kCells * 16) / 16; i += kWgThreads)
       reinterpret_cast<uint4 *>(wsm)[i] = make_uint4(0u, 0u, 0u, 0u);
-   }
    unsigned short *at = reinterpret_cast<unsigned short *>(wsm + kFirst + 2 * kCells * 16);
    if (tid < kSmThreads) slab_index(at, tid);
    unsigned short *tab = at + kCells;
