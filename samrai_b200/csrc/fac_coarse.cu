@@ -17,7 +17,9 @@
 // CTA's mbarrier of the colour, and a CTA goes on once its own threads have
 // met and its copies of the colour have come in.  A CTA cannot run ahead into
 // a copy that is still read: the value it sends next needs the values of the
-// cells that read it.  The sweep check goes round the cluster behind the
+// cells that read it.  Nor can a colour's phase complete while a thread still
+// waits for the one before: it is armed behind the block barrier after those
+// waits.  The sweep check goes round the cluster behind the
 // sweep: the CTAs of the checked patch store the outcome in every CTA, all
 // arrive at the cluster barrier after the black pass, and wait for it after
 // the next red pass, which is undone (each thread keeps its old red values)
@@ -303,6 +305,14 @@ k_coarse_solve(const CoarseCta *__restrict__ ctas, const CoarseCell *__restrict_
          int hit = 0;
          if (col == 1 && tol >= 0.0 && ct.last) hit = __syncthreads_or(any);
          else __syncthreads();
+         // Every thread has left its wait for the other colour's copies, so that
+         // colour's next phase may complete from here on: its bytes are expected
+         // now (early ones are counted already).  Expected any sooner, a thread that
+         // is late at its wait, one without a cell on the cut among them, could
+         // find the phase after the one it waits for complete, and wait for good:
+         // the other CTAs need nothing of it to send again.
+         if (tid == 0 && ct.nin[1 - col] && (col == 1 || sw > 0))
+            expect_bytes(bar0 + 8u * (1 - col), 8u * ct.nin[1 - col]);
          if (ncta == 1) {
             ghosts(col);
             if (col == 1) going = tol < 0.0 || hit;
@@ -318,8 +328,6 @@ k_coarse_solve(const CoarseCta *__restrict__ ctas, const CoarseCell *__restrict_
          ghosts(col);
          if (ct.nin[col]) {
             if (!dead) dead = !wait_bytes(bar0 + 8u * col, sw & 1);
-            // the next phase's bytes; early ones are counted already
-            if (tid == 0) expect_bytes(bar0 + 8u * col, 8u * ct.nin[col]);
          }
          if (col == 0 && sw > 0) {
             cluster_wait();
