@@ -435,14 +435,14 @@ int fac_time_interpolate(int dim, const fac_time_box *boxes, int nboxes,
                          void *stream);
 
 /* ---- bounded device waits (no counterpart in the reference).
- * The staged colour pass's consumer warps wait for each unit's copies at
- * most limit_cycles SM clock cycles (default 4e9, about 2 s) and then set
- * the context's device error flag, which the next norm or solve reports as
- * FAC_ERR_CUDA; every copy a block issued lands before the block exits, so
- * the context stays usable.  never = 1 makes that wait be for a phase no
- * copy completes: a test of the bound that ends with the error.
- * The coarsest solve's wait for the values of its cluster's other blocks has
- * the default limit and reports the same way.
+ * The staged passes' consumer warps wait for each unit's copies, and the
+ * threads of the coarsest solve for the values of their cluster's other
+ * blocks, at most limit_cycles SM clock cycles (default 4e9, about 2 s) and
+ * then set the context's device error flag, which the next norm or solve
+ * reports as FAC_ERR_CUDA; every copy into a block lands before the block
+ * exits, so the context stays usable.  never = 1 makes that wait be for a
+ * phase no copy completes (in the coarsest solve of an even-numbered problem
+ * for one thread alone): a test of the bound that ends with the error.
  * fac_clear_device_error resets the flag. */
 int fac_set_wait_test(fac_ctx *ctx, long long limit_cycles, int never);
 int fac_clear_device_error(fac_ctx *ctx);

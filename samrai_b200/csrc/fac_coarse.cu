@@ -25,6 +25,13 @@
 // the next red pass, which is undone (each thread keeps its old red values)
 // if the sweep before it was the last.
 //
+// A thread whose wait runs out sets the device error flag and goes on without
+// waiting, so that every CTA still sends, and arrives at the cluster barrier,
+// as often as the others; the sweep's outcome carries the stop to all of them.
+// Thread 0, which arms the phases, then waits for the values still on their way
+// before its CTA exits.  (The cluster barrier itself is the hardware's, between
+// CTAs that are resident together: it opens because every thread arrives.)
+//
 // The homogeneous Robin values behind physical faces are a list of their own,
 // renewed while the copies are on their way, one division per thread.
 //
@@ -87,10 +94,8 @@ __device__ __forceinline__ void expect_bytes(unsigned bar, unsigned bytes)
 }
 
 // Wait for a phase of an mbarrier whose bytes come from other CTAs; gives up
-// after kCoarseWaitCycles.
-constexpr long long kCoarseWaitCycles = 4000000000ll;
-
-__device__ __forceinline__ bool wait_bytes(unsigned bar, unsigned parity)
+// after `limit` SM clock cycles.
+__device__ __forceinline__ bool wait_bytes(unsigned bar, unsigned parity, long long limit)
 {
    unsigned ok = 0;
    long long t0 = 0;
@@ -106,7 +111,7 @@ __device__ __forceinline__ bool wait_bytes(unsigned bar, unsigned parity)
          : "memory");
       if (ok) return true;
       if (n == 0) t0 = clock64();
-      else if (clock64() - t0 > kCoarseWaitCycles) return false;
+      else if (clock64() - t0 > limit) return false;
    }
 }
 
@@ -137,12 +142,14 @@ k_coarse_solve(const CoarseCta *__restrict__ ctas, const CoarseCell *__restrict_
                double *__restrict__ u, const double *__restrict__ f,
                const double *__restrict__ dside, const double *__restrict__ cfield,
                double dconst, double cconst, BcCoefs bc, int ncta, int nsweeps, double tol,
-               int *__restrict__ run, long long *__restrict__ sweeps, int *__restrict__ err)
+               int *__restrict__ run, long long *__restrict__ sweeps, int *__restrict__ err,
+               WaitTest wt)
 {
    extern __shared__ __align__(16) double su[];
-   __shared__ unsigned long long bars[2];
+   __shared__ unsigned long long bars[3];  // per colour, and one that nothing completes
    __shared__ double bnum[6], bden[6], binv[6];
-   __shared__ int flag[2];
+   // the outcome of a sweep, by its parity: {some residual above tol, a wait ran out}
+   __shared__ __align__(8) int2 flag[2];
    pdl_begin();
    const CoarseCta ct = ctas[blockIdx.x];
    if (!run[ct.prob]) return;  // the whole cluster
@@ -177,8 +184,8 @@ k_coarse_solve(const CoarseCta *__restrict__ ctas, const CoarseCell *__restrict_
       }
    }
    if (tid == 0) {
-      flag[0] = flag[1] = 0;
-      for (int k = 0; k < 2; ++k)
+      flag[0] = flag[1] = make_int2(0, 0);
+      for (int k = 0; k < 3; ++k)
          asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8u * k) : "memory");
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       for (int k = 0; k < 2; ++k)
@@ -255,7 +262,16 @@ k_coarse_solve(const CoarseCta *__restrict__ ctas, const CoarseCell *__restrict_
    ghosts(0);
    ghosts(1);
    __syncthreads();
-   bool going = true, dead = false;
+   // the test of the bounded wait: in problems of even number the last thread
+   // of the first CTA waits for what nothing completes, in the others every
+   // thread does
+   const bool never = wt.never && ((ct.prob & 1) || (ct.rank == 0 && tid == kCoarseThreads - 1));
+   bool going = true;
+   int dead = 0;  // 1 + 2 sweep + colour of this thread's wait that ran out
+   auto outcome = [&](int s) {
+      const long long v = *(volatile long long *)&flag[s & 1];
+      return (tol < 0.0 || (int)v != 0) && (int)(v >> 32) == 0;
+   };
    int sw = 0;
    for (; sw < nsweeps; ++sw) {
       bool any = false;
@@ -311,7 +327,7 @@ k_coarse_solve(const CoarseCta *__restrict__ ctas, const CoarseCell *__restrict_
          // is late at its wait, one without a cell on the cut among them, could
          // find the phase after the one it waits for complete, and wait for good:
          // the other CTAs need nothing of it to send again.
-         if (tid == 0 && ct.nin[1 - col] && (col == 1 || sw > 0))
+         if (tid == 0 && !dead && ct.nin[1 - col] && (col == 1 || sw > 0))
             expect_bytes(bar0 + 8u * (1 - col), 8u * ct.nin[1 - col]);
          if (ncta == 1) {
             ghosts(col);
@@ -321,17 +337,23 @@ k_coarse_solve(const CoarseCta *__restrict__ ctas, const CoarseCell *__restrict_
          if (col == 1) {
             // the last sweep's outcome was read by all after the red pass; no
             // CTA stores into its place again before it has seen this arrival
-            if (tid == 0 && sw > 0) flag[(sw - 1) & 1] = 0;
-            if (hit && tid < ncta) store_remote(map_rank(flag0 + 4u * (sw & 1), tid), 1);
+            if (tid == 0 && sw > 0) flag[(sw - 1) & 1] = make_int2(0, 0);
+            if (hit && tid < ncta) store_remote(map_rank(flag0 + 8u * (sw & 1), tid), 1);
+            if (dead)
+               for (int r = 0; r < ncta; ++r) store_remote(map_rank(flag0 + 8u * (sw & 1) + 4u, r), 1);
             cluster_arrive();
          }
          ghosts(col);
-         if (ct.nin[col]) {
-            if (!dead) dead = !wait_bytes(bar0 + 8u * col, sw & 1);
+         if (ct.nin[col] && !dead &&
+             !wait_bytes(never ? bar0 + 16u : bar0 + 8u * col, never ? 0u : sw & 1, wt.limit)) {
+            // on with the passes, without waiting: every CTA keeps sending and
+            // arriving until the outcome of a sweep stops them all together
+            dead = 1 + 2 * sw + col;
+            atomicExch(err, 1);
          }
          if (col == 0 && sw > 0) {
             cluster_wait();
-            if (tol >= 0.0) going = *(volatile int *)&flag[(sw - 1) & 1] != 0;
+            going = outcome(sw - 1);
             if (!going) {
                // the sweep before was the last: take this red pass back
 #pragma unroll
@@ -349,11 +371,25 @@ k_coarse_solve(const CoarseCta *__restrict__ ctas, const CoarseCell *__restrict_
       }
       if (!going) break;
    }
+   // passes of each colour all CTAs have made: a stop comes after a red one
+   const int made[2] = {sw < nsweeps ? sw + 1 : sw, sw};
    if (ncta > 1 && going && sw > 0) {
       cluster_wait();
-      if (tol >= 0.0) going = *(volatile int *)&flag[(sw - 1) & 1] != 0;
+      going = outcome(sw - 1);
    }
-   if (dead && tid == 0) atomicExch(err, 1);
+   // Values on their way into this CTA's shared memory land before it exits.
+   // Thread 0 has seen every phase of both colours complete or, where its own
+   // wait ran out, goes through those since then now; the first of them is armed.
+   if (dead && tid == 0) {
+      const int gsw = (dead - 1) >> 1, gcol = (dead - 1) & 1;
+      for (int col = 0; col < 2; ++col) {
+         const int first = col < gcol ? gsw + 1 : gsw;
+         for (int q = first; ct.nin[col] && q < made[col]; ++q) {
+            if (q > first) expect_bytes(bar0 + 8u * col, 8u * ct.nin[col]);
+            if (!wait_bytes(bar0 + 8u * col, q & 1, WaitTest().limit)) break;
+         }
+      }
+   }
 #pragma unroll
    for (int col = 0; col < 2; ++col) {
       const int self0 = col ? ct.ncol[0] : 0;
@@ -378,7 +414,7 @@ k_coarse_solve(const CoarseCta *__restrict__ ctas, const CoarseCell *__restrict_
 using CoarseFn = void (*)(const CoarseCta *, const CoarseCell *, const long long *,
                           const unsigned *, const unsigned *, const PatchDesc *, double *,
                           const double *, const double *, const double *, double, double, BcCoefs,
-                          int, int, double, int *, long long *, int *);
+                          int, int, double, int *, long long *, int *, WaitTest);
 
 template <int DIM, bool DVAR, int CKIND>
 CoarseFn pick_sp(int sp)
@@ -461,7 +497,8 @@ cudaError_t launch_coarse_solve(cudaStream_t s, int dim, const PoissonSpec &spec
                                 const unsigned *push, const unsigned *ghost,
                                 const PatchDesc *patches, double *u, const double *f,
                                 const double *dside, const double *cfield, const BcCoefs &bc,
-                                int nsweeps, double tol, int *run, long long *sweeps, int *err)
+                                int nsweeps, double tol, int *run, long long *sweeps, int *err,
+                                const WaitTest &wt)
 {
    if (nprob <= 0 || nsweeps <= 0) return cudaSuccess;
    cudaLaunchAttribute attr[2];
@@ -469,7 +506,7 @@ cudaError_t launch_coarse_solve(cudaStream_t s, int dim, const PoissonSpec &spec
    add_kernel_launches(1);
    return cudaLaunchKernelEx(&cfg, pick(dim, spec, sp), ctas, cells, halo, push, ghost, patches,
                              u, f, dside, cfield, spec.d_const, spec.c_const, bc, ncta, nsweeps,
-                             tol, run, sweeps, err);
+                             tol, run, sweeps, err, wt);
 }
 
 }  // namespace samrai_b200

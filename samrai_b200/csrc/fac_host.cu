@@ -434,7 +434,7 @@ struct fac_ctx {
    int stage_budget = 32 * 1024;  // shared memory of one stage (unit) of the staged pass
    int stage_depth = 2;           // stages per CTA of the staged pass
    DevArray<int> kerr;       // set by kernels whose bounded waits ran out
-   WaitTest wait_test;       // bound of the staged pass's waits (fac_set_wait_test)
+   WaitTest wait_test;       // bound of the kernels' waits (fac_set_wait_test)
    // Robin coefficients varying along the boundary (fac_set_bc_faces);
    // while any are set the colour passes take the fill-based path, whose
    // boundary fills read them
@@ -2641,7 +2641,7 @@ void smooth(fac_ctx *c, int fid_e, int fid_r, int ln, int nsweeps, double tol)
          reinterpret_cast<const long long *>(t + L.coarse_at[0]),
          reinterpret_cast<const unsigned *>(t + L.coarse_at[3]),
          reinterpret_cast<const unsigned *>(t + L.coarse_at[4]), L.d_patches.p, e, r, L.d.p, L.c.p,
-         c->bc, nsweeps, tol, c->run.p, c->sweeps_call.p, c->kerr.p));
+         c->bc, nsweeps, tol, c->run.p, c->sweeps_call.p, c->kerr.p, c->wait_test));
       prof_end(c, pi);
    }
    for (int isweep = 0; isweep < (one_launch ? 0 : nsweeps); ++isweep) {

@@ -148,10 +148,11 @@ struct BcCoefs {
    int face_nprob = 0;
 };
 
-// The staged colour pass's wait for a unit's copies: it gives up after
-// `limit` SM clock cycles (about 2 s by default).  never = 1 is the test of
-// that bound: the wait is on an mbarrier nothing arrives on, so it runs
-// out (the stage's copies still land before the block exits).
+// The staged passes' wait for a unit's copies and the coarsest solve's for the
+// values of its cluster's other CTAs: they give up after `limit` SM clock
+// cycles (about 2 s by default).  never = 1 is the test of that bound: the wait
+// is on an mbarrier nothing arrives on, so it runs out (what is on its way into
+// a block still lands before the block exits).
 struct WaitTest {
    long long limit = 4000000000ll;
    int never = 0;

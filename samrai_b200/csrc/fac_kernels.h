@@ -121,7 +121,8 @@ cudaError_t launch_coarse_solve(cudaStream_t s, int dim, const PoissonSpec &spec
                                 const unsigned *push, const unsigned *ghost,
                                 const PatchDesc *patches, double *u, const double *f,
                                 const double *dside, const double *cfield, const BcCoefs &bc,
-                                int nsweeps, double tol, int *run, long long *sweeps, int *err);
+                                int nsweeps, double tol, int *run, long long *sweeps, int *err,
+                                const WaitTest &wt = WaitTest());
 // Ghost fill from a gather list of n elements (copies and constant refines,
 // see k_fill_gather) plus the physical-boundary items of the same fill.
 template <class T>

@@ -1,12 +1,12 @@
 """Bounded device waits.
 
 Every wait of the staged colour pass (a unit's copies landing in shared
-memory, a stage coming free) gives up after a bound and sets the context's
-device error flag instead of hanging the GPU; the next norm reports
-FAC_ERR_CUDA and the context stays usable.  Here the consumer warps are made
-to wait on an mbarrier nothing arrives on, with a 1e6-cycle bound: the pass
-must end with the error, and after the flag is cleared the same context must
-smooth exactly like the oracle again.
+memory, a stage coming free) and of the coarsest solve (another block's values)
+gives up after a bound and sets the context's device error flag instead of
+hanging the GPU; the next norm reports FAC_ERR_CUDA and the context stays
+usable.  Here they are made to wait on an mbarrier nothing arrives on, with a
+1e6-cycle bound: the call must end with the error, and after the flag is
+cleared the same context must smooth exactly as before.
 """
 import numpy as np
 import pytest
@@ -48,3 +48,54 @@ def test_bounded_wait_runs_out_and_context_recovers(require_gpu):
     assert np.array_equal(g.download(E, 0, ln), o.get(E, ln))
     g.rms_norm(R)
     g.close()
+
+
+@pytest.mark.parametrize("nprob", [1, 2])
+@pytest.mark.parametrize("nx", [64, 97])
+def test_coarsest_solve_wait_runs_out(nprob, nx, require_gpu):
+    """One launch of several blocks per problem.  In problem 0 a single thread
+    (not the one that arms the mbarriers) gives up, in problem 1 every thread:
+    the flag is set, all blocks stop together long before the last sweep, and
+    the context then solves like one that never failed."""
+    def problem():
+        return configs.Problem(dim=2, n0=(nx, nx, 1), xlo=(0.0,) * 3, xup=(1.0,) * 3,
+                               levels=[configs.Level((1, 1, 1), np.array(
+                                   [[0, 0, 0, nx - 1, nx - 1, 0]], dtype=np.int32))])
+
+    rng = np.random.default_rng(nx)
+    data = [{fid: rng.standard_normal(configs.field_size(problem(), 0, 1 if fid == E else 0))
+             for fid in (E, R)} for _ in range(nprob)]
+
+    def fresh():
+        ctx = fac.FacContext([problem() for _ in range(nprob)])
+        load(ctx)
+        return ctx
+
+    def load(ctx):
+        for i, d in enumerate(data):
+            for fid in (E, R):
+                ctx.upload(fid, i, 0, d[fid])
+
+    sweeps = 200
+    a, b = fresh(), fresh()
+    n0 = fac.kernel_launches()
+    want = b.smooth(E, R, 0, sweeps, 1e-300)
+    assert fac.kernel_launches() - n0 < sweeps  # all sweeps in one launch
+    assert np.all(want == sweeps)
+    L = fac.load_library()
+    for _ in range(2):
+        assert L.fac_set_wait_test(a.h, 1_000_000, 1) == 0
+        # the first wait runs out in sweep 0, whose outcome stops sweep 1
+        assert np.all(a.smooth(E, R, 0, sweeps, 1e-300) == 1)
+        with pytest.raises(fac.FacError) as err:
+            a.rms_norm(R)
+        assert err.value.code == FAC_ERR_CUDA
+        assert L.fac_set_wait_test(a.h, 4_000_000_000, 0) == 0
+        assert L.fac_clear_device_error(a.h) == 0
+        load(a)
+        assert np.array_equal(a.smooth(E, R, 0, sweeps, 1e-300), want)
+        a.rms_norm(R)
+        for i in range(nprob):
+            assert np.array_equal(a.download(E, i, 0), b.download(E, i, 0))
+    a.close()
+    b.close()
