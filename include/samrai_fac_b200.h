@@ -438,8 +438,8 @@ int fac_time_interpolate(int dim, const fac_time_box *boxes, int nboxes,
  * The staged passes' consumer warps wait for each unit's copies, and the
  * threads of the coarsest solve for the values of their cluster's other
  * blocks, at most limit_cycles SM clock cycles (default 4e9, about 2 s) and
- * then set the context's device error flag, which the next norm or solve
- * reports as FAC_ERR_CUDA; every copy into a block lands before the block
+ * then set the context's device error flag, which the next norm, dot
+ * product or solve reports as FAC_ERR_CUDA; every copy into a block lands before the block
  * exits, so the context stays usable.  never = 1 makes that wait be for a
  * phase no copy completes (in the coarsest solve of an even-numbered problem
  * for one thread alone): a test of the bound that ends with the error.

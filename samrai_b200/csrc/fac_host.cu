@@ -2847,14 +2847,21 @@ void reduce_launch(fac_ctx *c, int mode, int fid_x, int fid_y)
 
 void rms_norm_launch(fac_ctx *c, int fid) { reduce_launch(c, kReduceNorm, fid, fid); }
 
+// The sums of the last reduction, once the stream has drained; throws when a
+// kernel before it set the device error flag.
+const double2 *reduce_read(fac_ctx *c)
+{
+   CUDA_CHECK(cudaStreamSynchronize(c->stream));
+   if (*c->back.err)
+      throw FacError(FAC_ERR_CUDA, "a bounded wait of a staged pass or of the coarsest solve "
+                                   "ran out (device error flag; fac_clear_device_error resets it)");
+   return c->back.acc;
+}
+
 void rms_norm_read(fac_ctx *c, std::vector<double> &out)
 {
    const int np = nprob(c);
-   CUDA_CHECK(cudaStreamSynchronize(c->stream));
-   if (*c->back.err)
-      throw FacError(FAC_ERR_CUDA, "a bounded wait of a staged colour pass or of the coarsest solve "
-                                   "ran out (device error flag; fac_clear_device_error resets it)");
-   const double2 *acc = c->back.acc;
+   const double2 *acc = reduce_read(c);
    out.resize(np);
    for (int p = 0; p < np; ++p) {
       const double num = std::sqrt(acc[p].x);
@@ -4157,8 +4164,7 @@ const double2 *vec_reduce(fac_ctx *c, int mode, int fid_x, int fid_y)
    vec_all_active(c);
    reduce_launch(c, mode, fid_x, fid_y);
    CUDA_CHECK(cudaGetLastError());
-   CUDA_CHECK(cudaStreamSynchronize(c->stream));
-   return c->back.acc;
+   return reduce_read(c);
 }
 
 }  // namespace

@@ -3,8 +3,8 @@
 Every wait of the staged colour pass (a unit's copies landing in shared
 memory, a stage coming free) and of the coarsest solve (another block's values)
 gives up after a bound and sets the context's device error flag instead of
-hanging the GPU; the next norm reports FAC_ERR_CUDA and the context stays
-usable.  Here they are made to wait on an mbarrier nothing arrives on, with a
+hanging the GPU; the next norm or dot product reports FAC_ERR_CUDA and the
+context stays usable.  Here they are made to wait on an mbarrier nothing arrives on, with a
 1e6-cycle bound: the call must end with the error, and after the flag is
 cleared the same context must smooth exactly as before.
 """
@@ -99,3 +99,27 @@ def test_coarsest_solve_wait_runs_out(nprob, nx, require_gpu):
             assert np.array_equal(a.download(E, i, 0), b.download(E, i, 0))
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("coarsest", [False, True])
+def test_composite_reductions_report_the_flag(coarsest, require_gpu):
+    """Every reduction over a field reports it, not the RMS norm alone."""
+    g = fac.FacContext([configs.config1() if coarsest else configs.small_3d(seed=7)])
+    L = fac.load_library()
+    assert L.fac_set_wait_test(g.h, 1_000_000, 1) == 0
+    if coarsest:
+        g.upload(R, 0, 0, np.ones(g.size(R, 0, 0)))
+        g.solve_coarsest()
+    else:
+        g.smooth(E, R, g.nlev - 1, 1)
+    for norm in (lambda: g.vec_l2_norm(R), lambda: g.vec_max_norm(R), lambda: g.vec_dot(R, E),
+                 lambda: g.rms_norm(R)):
+        with pytest.raises(fac.FacError) as err:
+            norm()
+        assert err.value.code == FAC_ERR_CUDA
+    assert L.fac_set_wait_test(g.h, 4_000_000_000, 0) == 0
+    assert L.fac_clear_device_error(g.h) == 0
+    g.vec_l2_norm(R)
+    g.vec_max_norm(R)
+    g.vec_dot(R, E)
+    g.close()
