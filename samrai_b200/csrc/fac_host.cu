@@ -1512,17 +1512,21 @@ bool build_coarse_tables(const fac_ctx *c, int ncta, int sp, CoarseTables &T)
          const Box &b = L.box[ip];
          const Box g = ghost_box(dim, b, 1);
          const long long gx = g.hi[0] - g.lo[0] + 1, gy = g.hi[1] - g.lo[1] + 1;
-         for (int a = 0; a < dim; ++a)
-            if (b.lo[a] < 0) return false;  // the colour rule below is that of k_rbgs for these
          for (int k = b.lo[2]; k <= b.hi[2]; ++k)
-            for (int j = b.lo[1]; j <= b.hi[1]; ++j)
+            for (int j = b.lo[1]; j <= b.hi[1]; ++j) {
+               // a row's colouring starts with the parity of this sum, by a division
+               // that rounds to zero (rb_slot, as in the reference's Fortran): in a
+               // row of a negative odd one both passes update the same cells
+               const int row = dim == 3 ? b.lo[0] + j + k : b.lo[1] + j;
+               if (row < 0 && (row & 1)) return false;
                for (int i = b.lo[0]; i <= b.hi[0]; ++i, ++q) {
                   where[q] = L.hp[ip].off1 + (i - g.lo[0]) + gx * ((j - g.lo[1]) + gy * (k - g.lo[2]));
                   ord[(size_t)(where[q] - base)] = q;
                   owner[q] = (int)((long long)q * ncta / N);
-                  colour[q] = (unsigned char)((dim == 3 ? i + j + k : i - b.lo[0] + b.lo[1] + j) & 1);
+                  colour[q] = (unsigned char)((i - b.lo[0] + row) & 1);
                   local[q] = ncol[2 * owner[q] + colour[q]]++;
                }
+            }
       }
       for (int v : ncol)
          if (v > kCoarseThreads * sp) return false;

@@ -87,3 +87,29 @@ def test_batch_of_sizes_stops_per_problem(require_gpu):
     assert np.array_equal(na, nb) and len(set(na.tolist())) > 1
     for x, y in zip(a, b):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("lo, n", [(-5, (64, 40)), (-4, (33, 97))])
+def test_negative_lower_index(lo, n, require_gpu):
+    """A 2-D level 0 may start below zero along x: one launch for all sweeps,
+    which are those of passes of a fixed count.  (Where the row sums that start
+    the colouring turn negative and odd, both passes update the same cells; such
+    levels keep to passes.)"""
+    p = _level0(2, n, (), False, 0, 0)
+    p.n0 = (n[0] + lo, n[1], 1)
+    p.levels = [configs.Level((1, 1, 1), np.array([[lo, 0, 0, n[0] + lo - 1, n[1] - 1, 0]],
+                                                  dtype=np.int32))]
+    rng = np.random.default_rng(2)
+    data = [(fid, rng.standard_normal(configs.field_size(p, 0, g))) for fid, g in ((E, 1), (R, 0))]
+    g = fac.FacContext([p])
+    g.set_staged(False)  # passes that take the Robin value of a face cell where they read it
+    sweeps, outs = 20, []
+    for tol in (1e-300, -1.0):
+        for fid, x in data:
+            g.upload(fid, 0, 0, x)
+        n0 = fac.kernel_launches()
+        assert g.smooth(E, R, 0, sweeps, tol)[0] == sweeps
+        outs.append((fac.kernel_launches() - n0, g.download(E, 0, 0)))
+    assert outs[0][0] < sweeps < outs[1][0]
+    assert np.array_equal(outs[0][1], outs[1][1])
+    g.close()
