@@ -390,6 +390,7 @@ struct LevelState {
    // level 0: the one-launch coarsest solve (build_coarse_solve); ncta = 0:
    // the level does not fit it
    int coarse_ncta = 0, coarse_sp = 0, coarse_smem = 0;
+   std::vector<double> coarse_bytes_prob;  // u, f, D, C in and u out, per problem
    DevArray<unsigned char> d_coarse;  // its tables, one after another
    size_t coarse_at[5] = {0, 0, 0, 0, 0};  // halo, CTAs, cells, pushes, ghosts
    DevArray<int> last_patch;
@@ -512,11 +513,12 @@ struct fac_ctx {
    std::vector<ProfRec> graph_prof;
    long long graph_launches = 0;
    bool graph_profiled = false;
+   static constexpr int kProfKinds = 7;
    struct KindAcc {
       long long n = 0;
       double ms = 0, bytes = 0;
    };
-   KindAcc graph_acc[6];
+   KindAcc graph_acc[kProfKinds];
    // per-operation wall time with a stream synchronisation on both sides
    // (tbox::Timer::barrierAndStart semantics, tbox/Timer.C:174)
    bool tracing = false;
@@ -1850,6 +1852,12 @@ void build_chunks(fac_ctx *c, int ln)
                                          (c->spec.d_variable ? 8.0 * dim * pn : 0.0) +
                                          (c->spec.c_kind == 2 ? 4.0 * pn : 0.0);
    }
+   // the one-launch coarsest solve: u, f, C and the faces' D in, u out
+   L.coarse_bytes_prob.assign(np, 0.0);
+   for (int p = 0; p < np; ++p)
+      L.coarse_bytes_prob[p] =
+         (c->spec.c_kind == 2 ? 32.0 : 24.0) * (double)(L.prob_off0[p + 1] - L.prob_off0[p]) +
+         (c->spec.d_variable ? 8.0 * (double)(L.prob_offs[p + 1] - L.prob_offs[p]) : 0.0);
    double gcells = 0;
    L.fill_bytes_prob.assign(np, 0.0);
    for (const FillItem &it : L.fill_nc.items) {
@@ -2636,7 +2644,8 @@ void smooth(fac_ctx *c, int fid_e, int fid_r, int ln, int nsweeps, double tol)
    // smoothing to a tolerance on the coarsest level: every sweep in one launch
    const bool one_launch = tol >= 0.0 && ln == 0 && fmap && L.coarse_ncta > 0;
    if (one_launch) {
-      const int pi = prof_begin(c, 0, L.rb_bytes_prob, 2.0 * nsweeps);
+      // its data is read and written once, whatever the number of sweeps
+      const int pi = prof_begin(c, 6, L.coarse_bytes_prob, 1.0);
       const unsigned char *t = L.d_coarse.p;
       CUDA_CHECK(launch_coarse_solve(
          c->stream, c->dim, c->spec, np, L.coarse_ncta, L.coarse_sp, L.coarse_smem,
@@ -5569,7 +5578,7 @@ int fac_profile_read(fac_ctx *ctx, int kind, long long *launches, double *ms, do
    return guarded([&] {
       check_ops(ctx);
       CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
-      if (kind < 0 || kind > 5) throw FacError(FAC_ERR_ARG, "profile kind out of range");
+      if (kind < 0 || kind >= fac_ctx::kProfKinds) throw FacError(FAC_ERR_ARG, "profile kind out of range");
       long long n = ctx->graph_acc[kind].n;
       double t = ctx->graph_acc[kind].ms, b = ctx->graph_acc[kind].bytes;
       for (const auto &r : ctx->prof) {

@@ -113,3 +113,27 @@ def test_negative_lower_index(lo, n, require_gpu):
     assert outs[0][0] < sweeps < outs[1][0]
     assert np.array_equal(outs[0][1], outs[1][1])
     g.close()
+
+
+def test_profile_keeps_the_one_launch_solve_apart(require_gpu):
+    """Its values stay on the chip: it is no colour pass over the level's
+    arrays, and its bytes do not grow with the sweeps."""
+    probs = [_level0(3, (8, 8, 8), (), True, 2, 0), _level0(3, (12, 8, 8), (), True, 2, 1)]
+    g = fac.FacContext(probs)
+    faces = sum(configs.side_size(p, 0) for p in probs)
+    cells = sum(configs.field_size(p, 0, 0) for p in probs)
+    for i, p in enumerate(probs):
+        g.upload(R, i, 0, np.ones(configs.field_size(p, 0, 0)))
+    for sweeps in (5, 50):
+        g.profile(True)
+        g.smooth(E, R, 0, sweeps, 1e-300)
+        n, ms, by = g.profile_read(6)
+        assert (n, by) == (1, 8.0 * (faces + 4 * cells)) and ms > 0.0
+        assert g.profile_read(0) == (0, 0.0, 0.0)
+        g.profile(True)
+        g.smooth(E, R, 0, sweeps, -1.0)
+        assert g.profile_read(6)[0] == 0 and g.profile_read(0)[0] == 2 * sweeps
+    g.profile(False)
+    with pytest.raises(fac.FacError):
+        g.profile_read(7)
+    g.close()
