@@ -322,7 +322,6 @@ struct LevelState {
    DevArray<long long> facemap;
    DevArray<int> pushmap;
    std::vector<int> pushmap_h;  // host copy (face masks of the staged units)
-   std::vector<long long> facemap_h;  // host copy, level 0 while its solve is built
    // side-array faces that carry a coarsened finer-level flux
    DevArray<unsigned char> fcmask;
    bool fused_ok = false;
@@ -1404,7 +1403,7 @@ void build_residual_fixups(fac_ctx *c, int ln)
 // pass; that is exact only when the neighbour has the other colour, which
 // holds for the global 3-D colouring and, in 2-D, when every patch of the
 // level starts on the same parity of ifirst+jfirst (2d.f:140-147).
-void build_facemap(fac_ctx *c, int ln)
+std::vector<long long> build_facemap(fac_ctx *c, int ln)
 {
    LevelState &L = c->L[ln];
    const int dim = c->dim;
@@ -1475,16 +1474,17 @@ void build_facemap(fac_ctx *c, int ln)
    }
    L.fused_ok = ok;
    L.facemap.upload(fmap, c->stream);
-   if (ln == 0) L.facemap_h = std::move(fmap);
    L.pushmap.upload(pmap, c->stream);
    L.pushmap_h = std::move(pmap);
    build_stage_units(c, ln);
+   return fmap;
 }
 
 // Tables of the one-launch coarsest solve (fac_coarse.cu) for ncta CTAs per
 // problem: each problem's level-0 cells, in patch and storage order, in ncta
 // equal runs.  False when a CTA would hold more than sp cells of one colour
-// per thread, or its shared values do not fit.
+// per thread, or its shared values do not fit.  facemap: the level's
+// (build_facemap).
 struct CoarseTables {
    std::vector<CoarseCta> ctas;
    std::vector<CoarseCell> cells;
@@ -1493,7 +1493,8 @@ struct CoarseTables {
    int smem = 0;
 };
 
-bool build_coarse_tables(const fac_ctx *c, int ncta, int sp, CoarseTables &T)
+bool build_coarse_tables(const fac_ctx *c, const std::vector<long long> &facemap, int ncta, int sp,
+                         CoarseTables &T)
 {
    const LevelState &L = c->L[0];
    const int dim = c->dim;
@@ -1578,7 +1579,7 @@ bool build_coarse_tables(const fac_ctx *c, int ncta, int sp, CoarseTables &T)
                   if (x[a] == (s ? n[a] - 1 : 0)) {
                      const int t = a == 0 ? x[1] + n[1] * x[2]
                                           : (a == 1 ? x[0] + n[0] * x[2] : x[0] + n[0] * x[1]);
-                     m = L.facemap_h[d.offo[a][s] + t];
+                     m = facemap[d.offo[a][s] + t];
                   }
                   int at = -1;
                   if (m >= 0) {
@@ -1717,7 +1718,7 @@ double coarse_pass_us(int dim, int ncta, int sp, double load)
    return base + cell * load;
 }
 
-void build_coarse_solve(fac_ctx *c)
+void build_coarse_solve(fac_ctx *c, const std::vector<long long> &facemap)
 {
    LevelState &L = c->L[0];
    L.coarse_ncta = 0;
@@ -1747,7 +1748,7 @@ void build_coarse_solve(fac_ctx *c)
                     [](const Choice &x, const Choice &y) { return x.cost < y.cost; });
    CoarseTables T;
    for (const Choice &ch : choices) {
-      if (!build_coarse_tables(c, ch.ncta, ch.sp, T)) continue;
+      if (!build_coarse_tables(c, facemap, ch.ncta, ch.sp, T)) continue;
       L.coarse_ncta = ch.ncta;
       L.coarse_sp = ch.sp;
       L.coarse_smem = T.smem;
@@ -1765,8 +1766,6 @@ void build_coarse_solve(fac_ctx *c)
       L.d_coarse.upload(all, c->stream);
       break;
    }
-   L.facemap_h.clear();
-   L.facemap_h.shrink_to_fit();
 }
 
 void build_chunks(fac_ctx *c, int ln)
@@ -2548,7 +2547,8 @@ void initialize(fac_ctx *c)
    for (int ln = 0; ln < c->nlev; ++ln) {
       build_fill_tables(c, ln);
       build_cf_faces(c, ln);
-      build_facemap(c, ln);
+      const std::vector<long long> facemap = build_facemap(c, ln);
+      if (ln == 0) build_coarse_solve(c, facemap);
       build_chunks(c, ln);
       build_dirichlet_index(c, ln);
       if (ln > 0) build_prolong_tables(c, ln);
@@ -2561,7 +2561,6 @@ void initialize(fac_ctx *c)
       build_res_units(c, ln);
       build_residual_fixups(c, ln);
    }
-   build_coarse_solve(c);
    validate_tables(c);
    for (int ln = 0; ln < c->nlev; ++ln) {
       LevelState &L = c->L[ln];
