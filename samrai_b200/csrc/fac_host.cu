@@ -533,7 +533,6 @@ struct fac_ctx {
    std::vector<WorkReg> work_regs;
    DevArray<WorkReg> d_work_regs;
    DevArray<long long> sweeps_call, sweeps_coarse;
-   DevArray<double2> norm_acc;
    // results of the last reduction in pinned memory the GPU writes: per
    // problem the two sums, and the device error flag
    struct HostBack {
@@ -1599,14 +1598,8 @@ bool build_coarse_tables(const fac_ctx *c, const std::vector<long long> &facemap
                         }
                         at = pass == 0 ? slot[w] : (int)ce.nb[fc];
                      }
-                  } else if (m == -2) {
-                     // not a cell of this level: the ghost value as it is
-                     if (pass == 0) {
-                        at = nown + (int)halo[r].size();
-                        halo[r].push_back(next);
-                     } else {
-                        at = ce.nb[fc];
-                     }
+                  } else if (m != -1) {
+                     return false;  // neither a cell of the level nor a physical boundary
                   } else if (pass == 0) {
                      ghost[2 * r + colour[q]].push_back((unsigned)fc << 16 | (unsigned)local[q]);
                      at = 0;
@@ -2579,7 +2572,6 @@ void initialize(fac_ctx *c)
    c->run.upload(ones, c->stream);
    c->sweeps_call.alloc(np);
    c->sweeps_coarse.alloc(np);
-   c->norm_acc.alloc(np);
    if (!g_dry) c->back.alloc(np);
    c->hist.assign(np, {});
    if (!g_dry) {
@@ -2839,8 +2831,8 @@ void prolong_correct(fac_ctx *c, int fid_src, int fid_dst, int dest_ln)
    CUDA_CHECK(cudaGetLastError());
 }
 
-// One reduction over all levels of fields x (and y) into norm_acc and, on the
-// host, into back (valid once the stream has drained).
+// One reduction over all levels of fields x (and y) into back, on the host
+// (valid once the stream has drained).
 void reduce_launch(fac_ctx *c, int mode, int fid_x, int fid_y)
 {
    ReduceLevels lv;
@@ -2853,7 +2845,7 @@ void reduce_launch(fac_ctx *c, int mode, int fid_x, int fid_y)
                       field_ghost(fid_y)};
       lv.first[ln + 1] = lv.first[ln] + (int)L.cell_chunks.size();
    }
-   launch_reduce(c->stream, c->dim, mode, lv, nprob(c), c->norm_acc.p, c->back.acc, c->kerr.p,
+   launch_reduce(c->stream, c->dim, mode, lv, nprob(c), c->back.acc, c->kerr.p,
                  c->back.err);
 }
 
@@ -3630,9 +3622,8 @@ void learned_precondition(fac_ctx *c, int vslot, int zslot)
    launch_alpha(c->stream, c->dot_acc.p, c->active.p, np, c->alpha.p);
    for (int l = 0; l < c->nlev; ++l) {
       LevelState &L = c->L[l];
-      launch_g1_to_g0<double>(c->stream, c->dim, (int)L.cell_chunks.size(), L.d_patches.p,
-                              L.d_cell_chunks.p, L.e.p, kry_vec(c, l, zslot), true,
-                              c->alpha.p);
+      launch_add_scaled(c->stream, c->dim, (int)L.cell_chunks.size(), L.d_patches.p,
+                        L.d_cell_chunks.p, L.e.p, kry_vec(c, l, zslot), c->alpha.p);
    }
    CUDA_CHECK(cudaGetLastError());
 }

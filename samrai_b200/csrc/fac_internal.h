@@ -480,7 +480,7 @@ constexpr int kCoarseClusterMax = 16;
 
 // One CTA: its own cells are cells[cell0 ..], the ncol[0] red ones first,
 // and its shared values are those cells, nhalo copies of cells other CTAs
-// own (or fixed ghost values), then the physical-boundary ghost values of its
+// own, then the physical-boundary ghost values of its
 // red and of its black cells.
 struct CoarseCta {
    int prob, patch0, rank;

@@ -1231,13 +1231,14 @@ k_reduce_partial(ReduceLevels lv)
 }
 
 // Per problem: each level's partials in chunk order (thread-strided, the same
-// tree), the levels added in level order; to acc[prob] and to the host (pinned
-// memory), with the device error flag.  A warp per level.
+// tree), the levels added in level order; to the host (pinned memory), with the
+// device error flag.  A warp per level.
 template <int MODE>
 __global__ void __launch_bounds__(kThreads)
-k_reduce_levels(ReduceLevels lv, double2 *__restrict__ acc, double2 *__restrict__ host,
-                const int *__restrict__ err, int *__restrict__ host_err)
+k_reduce_levels(ReduceLevels lv, double2 *__restrict__ host, const int *__restrict__ err,
+                int *__restrict__ host_err)
 {
+   static_assert(kMaxLevels <= kThreads / 32, "a warp per level");
    pdl_begin();
    __shared__ double rs[kMaxLevels][kThreads], rv[kMaxLevels][kThreads];
    __shared__ double2 sum[kMaxLevels];
@@ -1264,7 +1265,6 @@ k_reduce_levels(ReduceLevels lv, double2 *__restrict__ acc, double2 *__restrict_
          a.x = MODE == kReduceMax ? fmax(a.x, sum[l].x) : a.x + sum[l].x;
          a.y += sum[l].y;
       }
-      acc[pr] = a;
       host[pr] = a;
       if (pr == 0) *host_err = *err;
    }
@@ -1872,12 +1872,12 @@ k_combine_dots(KryLevels lv, const double *__restrict__ a, int K,
    }
 }
 
-// dst (ghost-0, FP64) = src interior (ghost-1)
-template <int DIM, class TS>
+// dst (ghost-0) += scale[problem] src interior (ghost-1)
+template <int DIM>
 __global__ void __launch_bounds__(kThreads)
-k_g1_to_g0(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ chunks, int nwork,
-           const TS *__restrict__ src, double *__restrict__ dst, int add,
-           const double *__restrict__ scale, double *__restrict__ dst1)
+k_add_scaled(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ chunks, int nwork,
+             const double *__restrict__ src, double *__restrict__ dst,
+             const double *__restrict__ scale)
 {
    pdl_begin();
    WORK_LOOP(ch) {
@@ -1891,17 +1891,15 @@ k_g1_to_g0(const PatchDesc *__restrict__ patches, const Chunk *__restrict__ chun
          const int i = p.lo[0] + ci;
          const int j = p.lo[1] + cj;
          const int k = DIM == 3 ? p.lo[2] + ck : 0;
-         const long long c1 = cidx<DIM>(p, p.off1, 1, i, j, k);
-         double v = (double)src[c1];
-         if (scale) v = scale[p.prob] * v;
-         dst[p.off0 + lin] = add ? dst[p.off0 + lin] + v : v;
-         if (dst1) dst1[c1] = v;
+         const double v = scale[p.prob] * src[cidx<DIM>(p, p.off1, 1, i, j, k)];
+         dst[p.off0 + lin] = dst[p.off0 + lin] + v;
       }
    }
 }
 
-// The same without scale over all levels in one launch, blocks per chunk as
-// ELEMENT_LOOP
+// dst (ghost-0, FP64) = src interior (ghost-1), also into the interior of a
+// ghost-1 dst1 where one is given, over all levels in one launch, blocks per
+// chunk as ELEMENT_LOOP
 template <int DIM, class TS>
 __global__ void __launch_bounds__(kThreads)
 k_store_levels(StoreLevels lv)
@@ -2068,22 +2066,16 @@ void launch_store_levels(cudaStream_t s, int dim, const StoreLevels &lv)
 template void launch_store_levels<double>(cudaStream_t, int, const StoreLevels &);
 template void launch_store_levels<float>(cudaStream_t, int, const StoreLevels &);
 
-template <class TS>
-void launch_g1_to_g0(cudaStream_t s, int dim, int nchunks, const PatchDesc *patches,
-                     const Chunk *chunks, const TS *src, double *dst, bool add,
-                     const double *scale, double *dst1)
+void launch_add_scaled(cudaStream_t s, int dim, int nchunks, const PatchDesc *patches,
+                       const Chunk *chunks, const double *src, double *dst, const double *scale)
 {
    if (nchunks <= 0) return;
    g_launches.fetch_add(1, std::memory_order_relaxed);
    if (dim == 2)
-      launch_after(k_g1_to_g0<2, TS>, split_grid(k_g1_to_g0<2, TS>, nchunks), kThreads, 0, s, patches, chunks, nchunks, src, dst, add ? 1 : 0, scale, dst1);
+      launch_after(k_add_scaled<2>, split_grid(k_add_scaled<2>, nchunks), kThreads, 0, s, patches, chunks, nchunks, src, dst, scale);
    else
-      launch_after(k_g1_to_g0<3, TS>, split_grid(k_g1_to_g0<3, TS>, nchunks), kThreads, 0, s, patches, chunks, nchunks, src, dst, add ? 1 : 0, scale, dst1);
+      launch_after(k_add_scaled<3>, split_grid(k_add_scaled<3>, nchunks), kThreads, 0, s, patches, chunks, nchunks, src, dst, scale);
 }
-template void launch_g1_to_g0<double>(cudaStream_t, int, int, const PatchDesc *, const Chunk *,
-                                      const double *, double *, bool, const double *, double *);
-template void launch_g1_to_g0<float>(cudaStream_t, int, int, const PatchDesc *, const Chunk *,
-                                     const float *, double *, bool, const double *, double *);
 
 void launch_add_combination(cudaStream_t s, int dim, int nchunks, const PatchDesc *patches,
                             const Chunk *chunks, double *u, const double *Z, long long zstride,
@@ -2484,12 +2476,12 @@ void launch_convert(cudaStream_t s, const S *src, D *dst, long long n)
 }
 
 void launch_reduce(cudaStream_t s, int dim, int mode, const ReduceLevels &lv, int nprob,
-                   double2 *acc, double2 *host, const int *err, int *host_err)
+                   double2 *host, const int *err, int *host_err)
 {
    const int n = lv.first[lv.n];
    g_launches.fetch_add(n > 0 ? 2 : 1, std::memory_order_relaxed);
 #define VP(D, M) launch_after(k_reduce_partial<D, M>, work_grid(k_reduce_partial<D, M>, n), kThreads, 0, s, lv)
-#define VR(M) launch_after(k_reduce_levels<M>, nprob, kThreads, 0, s, lv, acc, host, err, host_err)
+#define VR(M) launch_after(k_reduce_levels<M>, nprob, kThreads, 0, s, lv, host, err, host_err)
    if (mode == kReduceDot) {
       if (n > 0) {
          if (dim == 2) VP(2, kReduceDot);

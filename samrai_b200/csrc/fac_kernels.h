@@ -89,13 +89,9 @@ bool launch_combine_dots(cudaStream_t s, const KryLevels &lv, const double *a, i
 // interior of a ghost-1 field (TS) into FP64 ghost-0 and ghost-1 fields
 template <class TS>
 void launch_store_levels(cudaStream_t s, int dim, const StoreLevels &lv);
-// dst (ghost-0) = interior of src (ghost-1), converted to FP64, times
-// scale[problem] when scale is given (with add: dst += it); with dst1 (a
-// ghost-1 FP64 field, not src) the same values also go to its interior
-template <class TS>
-void launch_g1_to_g0(cudaStream_t s, int dim, int nchunks, const PatchDesc *patches,
-                     const Chunk *chunks, const TS *src, double *dst, bool add = false,
-                     const double *scale = nullptr, double *dst1 = nullptr);
+// dst (ghost-0) += scale[problem] times the interior of src (ghost-1)
+void launch_add_scaled(cudaStream_t s, int dim, int nchunks, const PatchDesc *patches,
+                       const Chunk *chunks, const double *src, double *dst, const double *scale);
 // u interior += sum_i y[p*K+i] Z_i
 void launch_add_combination(cudaStream_t s, int dim, int nchunks, const PatchDesc *patches,
                             const Chunk *chunks, double *u, const double *Z, long long zstride,
@@ -215,8 +211,14 @@ void launch_add_interior(cudaStream_t s, int dim, int nchunks, const PatchDesc *
 template <class S, class D>
 void launch_convert(cudaStream_t s, const S *src, D *dst, long long n);
 
+// Composite-vector reduction over the interior cells of every level of lv, per
+// problem: kReduceNorm (sum w x x, sum w), kReduceDot (sum w x y, sum w),
+// kReduceMax (the largest |x| where w > 0, -).  The results go to host[problem]
+// and the device error flag *err to *host_err, both pinned host memory, valid
+// once the stream has drained.
 void launch_reduce(cudaStream_t s, int dim, int mode, const ReduceLevels &lv, int nprob,
-                   double2 *acc, double2 *host, const int *err, int *host_err);
+                   double2 *host, const int *err, int *host_err);
+// z = a[problem] x + b[problem] y on interior cells of one level
 void launch_vec_lincomb(cudaStream_t s, int dim, int nchunks, const PatchDesc *patches,
                         const Chunk *chunks, double *z, int zg, const double *x, int xg,
                         const double *y, int yg, const double *a, const double *b);
