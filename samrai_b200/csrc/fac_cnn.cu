@@ -609,6 +609,10 @@ k_conv_one(const float *__restrict__ v, const float *__restrict__ w, __nv_bfloat
             b[ks][j][h] = *reinterpret_cast<const uint32_t *>(&p);
          }
       }
+   // the taps from 27 on (of this lane: 24 + 2 q, 25 + 2 q) read the zero at index
+   // 0: a cell's own value in their place, times the weight 0, would make an
+   // infinite one a NaN
+   const int in0 = 24 + 2 * q < T ? -1 : 0, in1 = 25 + 2 * q < T ? -1 : 0;
    const long long nslab = nsamp * kTcSlabs;
    for (long long slab = blockIdx.x; slab < nslab; slab += gridDim.x) {
       const long long smp = slab / kTcSlabs;
@@ -620,6 +624,8 @@ k_conv_one(const float *__restrict__ v, const float *__restrict__ w, __nv_bfloat
       for (int st = warp; st < kSlabSteps; st += kSmWarps) {
          const int r0 = 16 * st + g, r1 = r0 + 8;
          const int p0 = at[r0], p1 = at[r1];
+         const int q0[2][2] = {{p0, p0}, {p0 & in0, p0 & in1}};  // of the upper taps of a step
+         const int q1[2][2] = {{p1, p1}, {p1 & in0, p1 & in1}};
          float d[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
          for (int k = 0; k < NSP; ++k)
@@ -627,8 +633,8 @@ k_conv_one(const float *__restrict__ v, const float *__restrict__ w, __nv_bfloat
             for (int ks = 0; ks < 2; ++ks) {
                const uint32_t a[4] = {pair(sv[k], p0 + off[ks][0], p0 + off[ks][1]),
                                       pair(sv[k], p1 + off[ks][0], p1 + off[ks][1]),
-                                      pair(sv[k], p0 + off[ks][2], p0 + off[ks][3]),
-                                      pair(sv[k], p1 + off[ks][2], p1 + off[ks][3])};
+                                      pair(sv[k], q0[ks][0] + off[ks][2], q0[ks][1] + off[ks][3]),
+                                      pair(sv[k], q1[ks][0] + off[ks][2], q1[ks][1] + off[ks][3])};
                mma_bf16(d[0], a, b[ks][0][0], b[ks][0][1]);
                mma_bf16(d[1], a, b[ks][1][0], b[ks][1][1]);
             }

@@ -137,3 +137,25 @@ def test_walks_of_several_slabs_match_fp64(n, require_gpu):
         r = w.grad.cpu().numpy().reshape(gr.shape)
         assert rel(gr, r) < 3e-2, rel(gr, r)
     net.close()
+
+
+@pytest.mark.parametrize("cell", [(9, 8, 7), (0, 0, 0), (17, 17, 17), (2, 0, 17), (3, 17, 0)])
+def test_infinite_input_reaches_the_output(cell, require_gpu):
+    """An infinite input is an infinite activation where its own tap is the
+    only positive one, and the positive layers after it spread it to the cells
+    within three of it; the others stay finite."""
+    import torch
+    net = fac.CNN(max_batch=1)
+    w1 = np.full((27, 16), -0.3, dtype=np.float32)
+    w1[13] = 0.5
+    net.set_weights([w1] + [np.full(s, 0.01, dtype=np.float32) for s in fac.CNN_SHAPES[1:]])
+    x = np.random.default_rng(3).random((1, S, S, S)).astype(np.float32)
+    x[(0,) + cell] = np.inf
+    xd = torch.from_numpy(x).cuda()
+    y = torch.zeros_like(xd)
+    net.forward(xd.data_ptr(), 1, y.data_ptr())
+    far = np.abs(np.indices((S, S, S)) - np.reshape(cell, (3, 1, 1, 1))).max(axis=0)
+    out = y.cpu().numpy()[0]
+    assert np.array_equal(out == np.inf, far <= 3)
+    assert np.isfinite(out[far > 3]).all()
+    net.close()
