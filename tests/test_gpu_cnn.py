@@ -159,3 +159,23 @@ def test_infinite_input_reaches_the_output(cell, require_gpu):
     assert np.array_equal(out == np.inf, far <= 3)
     assert np.isfinite(out[far > 3]).all()
     net.close()
+
+
+def test_largest_output_gradients_stay_finite(require_gpu):
+    """An output gradient beyond the largest BF16 number (3.39e38), which is a
+    sum of three of them: the gradients are those of a 2^-20 times smaller one,
+    scaled (1e-5: the order of the blocks' FP32 sums)."""
+    import torch
+    net = fac.CNN(max_batch=1)
+    net.set_weights([np.full(s, 1e-3, dtype=np.float32) for s in fac.CNN_SHAPES])
+    xd = torch.rand((1, S, S, S), generator=torch.Generator().manual_seed(1)).cuda()
+    md = torch.zeros_like(xd)
+    md[0, 9, 8, 7] = 1.0
+    gs = []
+    for scale in (1.0, 2.0 ** -20):
+        td = -1.7e38 * scale * md
+        gs.append(net.gradients(xd.data_ptr(), td.data_ptr(), md.data_ptr(), 1)[1])
+    for g, h in zip(*gs):
+        assert np.isfinite(g).all() and np.abs(g).max() > 0
+        assert np.allclose(g * 2.0 ** -20, h, rtol=1e-5, atol=1e-5 * np.abs(h).max())
+    net.close()
