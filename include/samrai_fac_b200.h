@@ -362,6 +362,10 @@ typedef struct fac_cnn fac_cnn;
 const char *fac_cnn_last_error(void);
 int fac_cnn_create(fac_cnn **net, int device, int max_batch, unsigned long long seed);
 int fac_cnn_destroy(fac_cnn *net);
+/* The bound of the tensor-core convolutions' waits for their multiplications
+ * and its test, as fac_set_wait_test below: a wait that runs out is reported as
+ * FAC_ERR_DEVICE by the call.  Clears the flag of an earlier one. */
+int fac_cnn_set_wait_test(fac_cnn *net, long long limit_cycles, int never);
 int fac_cnn_set_weights(fac_cnn *net, const float *w1, const float *w2,
                         const float *w3, const float *w4);
 int fac_cnn_get_weights(fac_cnn *net, float *w1, float *w2, float *w3,

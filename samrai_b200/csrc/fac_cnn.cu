@@ -38,6 +38,8 @@
 
 namespace {
 
+using samrai_b200::WaitTest;
+
 constexpr int S = FAC_CNN_BOX;       // sample box side (patch + halo)
 constexpr int S3 = S * S * S;
 constexpr int C = 16;                // hidden channels
@@ -122,9 +124,6 @@ static_assert(kTcBox % 4 == 0 && kTcRows % 4 == 0, "barriers aligned");
 template <unsigned N>
 constexpr unsigned kTcIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) |
                               ((128u >> 4) << 24);
-// a wait gives up after this many SM cycles (about 2 s)
-constexpr long long kTcWaitCycles = 4000000000ll;
-
 __device__ __forceinline__ unsigned tc_smem(const void *p)
 {
    return (unsigned)__cvta_generic_to_shared(p);
@@ -250,13 +249,14 @@ __device__ __forceinline__ void put_half(const float *o, __nv_bfloat16 *y, const
 // wt: BF16 B operands [(y, z) shift][input-channel half][N][8 in]; N = 48,
 // column (x tap, output channel), mode 0: y = relu(acc); mode 1: y = acc *
 // (gate > 0).  N = 16 (layer 4): columns 0..2 the x taps of the one output
-// channel, yf in FP32.  A wait that runs out sets *err and ends the CTA's
-// work.
+// channel, yf in FP32.  A wait that runs out sets *err and ends the CTA's work
+// once the multiplications in flight are done (a second wait, bounded too).
 template <int N>
 __global__ void __launch_bounds__(kTcThreads, 1)
 k_conv_mid_tc(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ wt,
               __nv_bfloat16 *__restrict__ y, const __nv_bfloat16 *__restrict__ gate,
-              float *__restrict__ yf, long long nsamp, int mode, int *__restrict__ err)
+              float *__restrict__ yf, long long nsamp, int mode, int *__restrict__ err,
+              WaitTest wait)
 {
    constexpr int NC = N == 48 ? 16 : 1;  // output channels
    extern __shared__ __align__(128) unsigned char tsm[];
@@ -265,7 +265,7 @@ k_conv_mid_tc(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restri
    unsigned short *tab = reinterpret_cast<unsigned short *>(edges + 2 * kTcEdge);
    unsigned short *rows = tab + kTcBox;  // cell of the slab of each output row
    unsigned long long *bar = reinterpret_cast<unsigned long long *>(rows + kTcRows);
-   unsigned *tslot = reinterpret_cast<unsigned *>(bar + 2);
+   unsigned *tslot = reinterpret_cast<unsigned *>(bar + 3);
    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
    for (int i = tid; i < kTcShifts * N * 2; i += kTcThreads)
       reinterpret_cast<uint4 *>(ws)[i] = reinterpret_cast<const uint4 *>(wt)[i];
@@ -273,7 +273,7 @@ k_conv_mid_tc(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restri
       reinterpret_cast<uint4 *>(tsm)[i] = make_uint4(0u, 0u, 0u, 0u);
    box_cells(tab, tid, kTcThreads);
    if (tid == 0) {
-      for (int i = 0; i < 2; ++i)
+      for (int i = 0; i < 3; ++i)  // one per half, and one that nothing completes
          asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(bar + i)) : "memory");
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
    }
@@ -304,11 +304,15 @@ k_conv_mid_tc(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restri
                  kTcReaders);
    };
    if (warp < kTcReadWarps && turns) stage(0);
+   // the mbarriers the readers wait on; a test's first wait is for the third's
+   // first phase
+   const unsigned bar_first = wait.never ? sb + 16u : sb, bar_step = wait.never ? 0u : 8u;
    bool ok = true;
+   int j = 0;
    // turn j multiplies half j % 2 of the CTA's slab j / 2, reads the half
    // before, and finishes the end rows of the slab read in the two turns before
    // that; an even turn also stages the next slab
-   for (int j = 0; turns && j < turns + 2; ++j) {
+   for (; turns && j < turns + 2; ++j) {
       // the slab is staged (the tensor cores read it through the async proxy),
       // the accumulators this turn writes are read, the end rows are there
       copies_done();
@@ -358,8 +362,8 @@ k_conv_mid_tc(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restri
          // the half before is multiplied (an mbarrier per half: one alone could be
          // a phase further already, with this turn's half)
          const long long t0 = clock64();
-         while (ok && !tc_try_wait(sb + 8u * ((j - 1) & 1), (unsigned)kr & 1u))
-            if (clock64() - t0 > kTcWaitCycles) ok = false;
+         while (ok && !tc_try_wait(bar_first + bar_step * ((j - 1) & 1), (unsigned)kr & 1u))
+            if (clock64() - t0 > wait.limit) ok = false;
          ok = __all_sync(0xffffffffu, ok);
          if (!ok) continue;  // leaves at the barrier
       }
@@ -438,7 +442,17 @@ k_conv_mid_tc(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restri
    copies_done();
    // every accumulator read is done before the tensor memory is released
    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-   if (!__syncthreads_and(ok) && tid == 0) atomicExch(err, 1);
+   if (!__syncthreads_and(ok) && tid == 0) {
+      atomicExch(err, 1);
+      // the last turn of each half may still be multiplying: its operands and
+      // accumulators stay until it is done
+      for (int t = j - 1; t >= 0 && t >= j - 2; --t) {
+         const long long t0 = clock64();
+         while (t < turns && !tc_try_wait(sb + 8u * (t & 1), (unsigned)(t >> 1) & 1u))
+            if (clock64() - t0 > WaitTest().limit) break;
+      }
+   }
+   __syncwarp();
    if (warp == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
@@ -915,6 +929,7 @@ struct fac_cnn {
    int *kerr = nullptr;                  // set by a tensor-core wait that ran out
    double *partial = nullptr;            // block sums of k_mask_sum
    unsigned *done = nullptr;
+   WaitTest wait_test;
    int sms = 0;
    int steps = 0;
    std::vector<void *> allocs;
@@ -969,7 +984,7 @@ void conv_mid(fac_cnn *n, const __nv_bfloat16 *x, const __nv_bfloat16 *wt, __nv_
               const __nv_bfloat16 *gate, long long nsamp, int mode, cudaStream_t st)
 {
    k_conv_mid_tc<48><<<slab_grid(n, nsamp, 1), kTcThreads, kTcSmem, st>>>(x, wt, y, gate, nullptr,
-                                                                         nsamp, mode, n->kerr);
+                                                                         nsamp, mode, n->kerr, n->wait_test);
 }
 
 void weight_mid(fac_cnn *n, const __nv_bfloat16 *x, const __nv_bfloat16 *dy, float *dw,
@@ -1002,7 +1017,7 @@ int forward_on(fac_cnn *n, const float *x, long long nsamp, cudaStream_t st, flo
    conv_mid(n, n->a[0], n->wf[0], n->a[1], nullptr, nsamp, 0, st);
    conv_mid(n, n->a[1], n->wf[1], n->a[2], nullptr, nsamp, 0, st);
    k_conv_mid_tc<16><<<slab_grid(n, nsamp, 1), kTcThreads, kTcSmem, st>>>(
-      n->a[2], n->wo, nullptr, nullptr, y, nsamp, 2, n->kerr);
+      n->a[2], n->wo, nullptr, nullptr, y, nsamp, 2, n->kerr, n->wait_test);
    samrai_b200::add_kernel_launches(4);
    CNN_CHECK(cudaGetLastError());
    return FAC_OK;
@@ -1173,6 +1188,19 @@ int fac_cnn_destroy(fac_cnn *n)
    cudaFreeHost(n->host);
    cudaStreamDestroy(n->stream);
    delete n;
+   return FAC_OK;
+}
+
+int fac_cnn_set_wait_test(fac_cnn *n, long long limit_cycles, int never)
+{
+   if (!n || limit_cycles < 1 || never < 0 || never > 1) {
+      t_cnn_error = "bad wait test";
+      return FAC_ERR_ARG;
+   }
+   n->wait_test.limit = limit_cycles;
+   n->wait_test.never = never;
+   CNN_CHECK(cudaMemsetAsync(n->kerr, 0, sizeof(int), n->stream));
+   CNN_CHECK(cudaStreamSynchronize(n->stream));
    return FAC_OK;
 }
 

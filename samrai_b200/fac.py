@@ -140,6 +140,7 @@ def load_library(build_if_missing=True):
         "fac_cnn_create": (ctypes.c_int, [ctypes.POINTER(vp), ctypes.c_int, ctypes.c_int,
                                           ctypes.c_ulonglong]),
         "fac_cnn_destroy": (ctypes.c_int, [vp]),
+        "fac_cnn_set_wait_test": (ctypes.c_int, [vp, ctypes.c_longlong, ctypes.c_int]),
         "fac_cnn_set_weights": (ctypes.c_int, [vp, fp, fp, fp, fp]),
         "fac_cnn_get_weights": (ctypes.c_int, [vp, fp, fp, fp, fp]),
         "fac_cnn_forward": (ctypes.c_int, [vp, vp, ctypes.c_longlong, vp]),

@@ -17,6 +17,7 @@ from oracle.oracle import E, Oracle, R
 pytestmark = pytest.mark.gpu
 
 FAC_ERR_CUDA = 3
+FAC_ERR_DEVICE = 6
 
 
 def test_bounded_wait_runs_out_and_context_recovers(require_gpu):
@@ -123,3 +124,26 @@ def test_composite_reductions_report_the_flag(coarsest, require_gpu):
     g.vec_max_norm(R)
     g.vec_dot(R, E)
     g.close()
+
+
+@pytest.mark.parametrize("n", [1, 60])
+def test_convolution_wait_runs_out(n, require_gpu):
+    """Batches of one slab a block and of several: the call reports the wait,
+    the blocks leave once their multiplications are done, and the network then
+    gives the bits of before."""
+    import torch
+    S = fac.CNN_BOX
+    net = fac.CNN(max_batch=n, seed=2)
+    x = torch.randn((n, S, S, S), generator=torch.Generator().manual_seed(n)).cuda()
+    want, y = torch.zeros_like(x), torch.zeros_like(x)
+    net.forward(x.data_ptr(), n, want.data_ptr())
+    L = fac.load_library()
+    for _ in range(2):
+        assert L.fac_cnn_set_wait_test(net.h, 1_000_000, 1) == 0
+        with pytest.raises(fac.FacError) as err:
+            net.forward(x.data_ptr(), n, y.data_ptr())
+        assert err.value.code == FAC_ERR_DEVICE
+        assert L.fac_cnn_set_wait_test(net.h, 4_000_000_000, 0) == 0
+        net.forward(x.data_ptr(), n, y.data_ptr())
+        assert torch.equal(y, want)
+    net.close()
