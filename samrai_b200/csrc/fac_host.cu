@@ -1498,22 +1498,42 @@ bool build_coarse_tables(const fac_ctx *c, const std::vector<long long> &facemap
    const LevelState &L = c->L[0];
    const int dim = c->dim;
    T = CoarseTables();
+   struct Ghost {
+      unsigned cell;  // of the CTA, red ones first
+      unsigned fc;
+   };
+   struct Push {
+      int cell, owner;  // of the problem's cells and the CTA that owns it
+      unsigned target;  // CTA rank << 16 | shared value there
+   };
+   std::vector<int> first(ncta + 1), local, seen, slot, pbase;
+   std::vector<unsigned char> colour;
+   std::vector<std::vector<long long>> halo(ncta);
+   std::vector<Ghost> ghost[2];
+   std::vector<Push> to;
    for (int p = 0; p < nprob(c); ++p) {
       const int pb = L.prob_patch_begin[p], pe = L.prob_patch_begin[p + 1];
-      const long long base = L.prob_off1[p];
-      long long N = 0;
-      for (int ip = pb; ip < pe; ++ip) N += L.box[ip].size();
-      // ordinal of every cell of the problem's slice of the ghost-1 field
-      std::vector<int> ord((size_t)(L.prob_off1[p + 1] - base), -1);
-      std::vector<int> owner((size_t)N), local((size_t)N);
-      std::vector<long long> where((size_t)N);  // ghost-1 element of each cell
-      std::vector<unsigned char> colour((size_t)N);
-      std::vector<int> ncol((size_t)ncta * 2, 0);
-      int q = 0;
+      // the problem's cells by ordinal: patch after patch, x fastest
+      pbase.assign(1, 0);
+      for (int ip = pb; ip < pe; ++ip) pbase.push_back(pbase.back() + (int)L.box[ip].size());
+      const int N = pbase.back();
+      // CTA r owns the ordinals from first[r] to first[r + 1]
+      for (int r = 0; r <= ncta; ++r) first[r] = (int)(((long long)r * N + ncta - 1) / ncta);
+      local.resize(N);
+      colour.resize(N);
+      const int cta0 = (int)T.ctas.size(), cells0 = (int)T.cells.size();
+      for (int r = 0; r < ncta; ++r) {
+         CoarseCta ct = {};
+         ct.prob = p;
+         ct.rank = r;
+         ct.patch0 = pb;
+         ct.cell0 = cells0 + first[r];
+         T.ctas.push_back(ct);
+      }
+      T.cells.resize((size_t)cells0 + N);
+      int q = 0, r = 0;
       for (int ip = pb; ip < pe; ++ip) {
          const Box &b = L.box[ip];
-         const Box g = ghost_box(dim, b, 1);
-         const long long gx = g.hi[0] - g.lo[0] + 1, gy = g.hi[1] - g.lo[1] + 1;
          for (int k = b.lo[2]; k <= b.hi[2]; ++k)
             for (int j = b.lo[1]; j <= b.hi[1]; ++j) {
                // a row's colouring starts with the parity of this sum, by a division
@@ -1522,125 +1542,136 @@ bool build_coarse_tables(const fac_ctx *c, const std::vector<long long> &facemap
                const int row = dim == 3 ? b.lo[0] + j + k : b.lo[1] + j;
                if (row < 0 && (row & 1)) return false;
                for (int i = b.lo[0]; i <= b.hi[0]; ++i, ++q) {
-                  where[q] = L.hp[ip].off1 + (i - g.lo[0]) + gx * ((j - g.lo[1]) + gy * (k - g.lo[2]));
-                  ord[(size_t)(where[q] - base)] = q;
-                  owner[q] = (int)((long long)q * ncta / N);
+                  while (q >= first[r + 1]) ++r;
                   colour[q] = (unsigned char)((i - b.lo[0] + row) & 1);
-                  local[q] = ncol[2 * owner[q] + colour[q]]++;
+                  local[q] = T.ctas[cta0 + r].ncol[colour[q]]++;
                }
             }
       }
-      for (int v : ncol)
-         if (v > kCoarseThreads * sp) return false;
+      for (r = 0; r < ncta; ++r)
+         for (int v : T.ctas[cta0 + r].ncol)
+            if (v > kCoarseThreads * sp) return false;
       // black cells after the red ones
-      for (int i = 0; i < (int)N; ++i)
-         if (colour[i]) local[i] += ncol[2 * owner[i]];
-      const int cta0 = (int)T.ctas.size();
-      std::vector<std::vector<CoarseCell>> mine(ncta);
-      std::vector<std::vector<long long>> halo(ncta);
-      // ghost values per CTA and colour: face << 16 | the cell's shared value
-      std::vector<std::vector<unsigned>> ghost(2 * ncta);
-      // CTAs a cell's value is pushed to: (rank, shared value there)
-      std::vector<std::vector<unsigned>> to((size_t)N);
-      std::vector<int> seen((size_t)N, -1), slot((size_t)N, 0);
-      for (int r = 0; r < ncta; ++r) {
-         mine[r].resize((size_t)ncol[2 * r] + ncol[2 * r + 1]);
-         CoarseCta ct = {};
-         ct.prob = p;
-         ct.rank = r;
-         ct.ncol[0] = ncol[2 * r];
-         ct.ncol[1] = ncol[2 * r + 1];
-         ct.patch0 = pb;
-         T.ctas.push_back(ct);
-      }
-      // first the copies a CTA needs and the ghost values of its red and black
-      // cells, then (their numbers known) where each ghost value is
-      std::vector<int> gnext(2 * ncta, 0);
-      for (int pass = 0; pass < 2; ++pass) {
-         q = 0;
-         for (int ip = pb; ip < pe; ++ip) {
-            const PatchDesc &d = L.hp[ip];
-            const Box &b = L.box[ip];
-            const int n[3] = {b.hi[0] - b.lo[0] + 1, b.hi[1] - b.lo[1] + 1, b.hi[2] - b.lo[2] + 1};
-            const long long step[3] = {1, n[0] + 2, (long long)(n[0] + 2) * (n[1] + 2)};
-            for (int lin = 0; lin < n[0] * n[1] * n[2]; ++lin, ++q) {
-               const int x[3] = {lin % n[0], lin / n[0] % n[1], lin / (n[0] * n[1])};
-               const int r = owner[q];
-               const int nown = ncol[2 * r] + ncol[2 * r + 1];
-               CoarseCell &ce = mine[r][local[q]];
-               ce.patch = ip;
-               ce.lin = lin;
-               if (ip == pe - 1) ce.last = (unsigned short)(T.ctas[cta0 + r].last = 1);
-               for (int fc = 0; fc < 2 * dim; ++fc) {
-                  const int a = fc >> 1, s = fc & 1;
-                  const long long next = where[q] + (s ? step[a] : -step[a]);
-                  long long m = next;
-                  if (x[a] == (s ? n[a] - 1 : 0)) {
-                     const int t = a == 0 ? x[1] + n[1] * x[2]
-                                          : (a == 1 ? x[0] + n[0] * x[2] : x[0] + n[0] * x[1]);
-                     m = facemap[d.offo[a][s] + t];
+      for (r = 0; r < ncta; ++r)
+         for (q = first[r]; q < first[r + 1]; ++q)
+            if (colour[q]) local[q] += T.ctas[cta0 + r].ncol[0];
+      // the copies a CTA needs and where each is pushed; cells are visited CTA by
+      // CTA, so seen and slot hold the present CTA's
+      seen.assign(N, -1);
+      slot.resize(N);
+      for (auto &h : halo) h.clear();
+      to.clear();
+      auto close = [&](int rank) {
+         // the ghost values are behind the copies, whose number is known now
+         CoarseCta &ct = T.ctas[cta0 + rank];
+         ct.nhalo = (int)halo[rank].size();
+         ct.ghost0 = (int)T.ghost.size();
+         int at = ct.ncol[0] + ct.ncol[1] + ct.nhalo;
+         for (int k = 0; k < 2; ++k) {
+            ct.nghost[k] = (int)ghost[k].size();
+            for (const Ghost &g : ghost[k]) {
+               T.ghost.push_back(g.fc << 16 | g.cell);
+               if (at > 0xffff) return false;
+               T.cells[(size_t)ct.cell0 + g.cell].nb[g.fc] = (unsigned short)at++;
+            }
+            ghost[k].clear();
+         }
+         return true;
+      };
+      q = r = 0;
+      for (int ip = pb; ip < pe; ++ip) {
+         const PatchDesc &d = L.hp[ip];
+         const Box &b = L.box[ip];
+         const int n[3] = {b.hi[0] - b.lo[0] + 1, b.hi[1] - b.lo[1] + 1, b.hi[2] - b.lo[2] + 1};
+         const int step[3] = {1, n[0], n[0] * n[1]};
+         const long long step1[3] = {1, n[0] + 2, (long long)(n[0] + 2) * (n[1] + 2)};
+         int x[3], lin = 0;
+         for (x[2] = 0; x[2] < n[2]; ++x[2])
+            for (x[1] = 0; x[1] < n[1]; ++x[1]) {
+               const bool inner = x[1] > 0 && x[1] < n[1] - 1 &&
+                                  (dim == 2 || (x[2] > 0 && x[2] < n[2] - 1));
+               for (x[0] = 0; x[0] < n[0]; ++x[0], ++lin, ++q) {
+                  while (q >= first[r + 1])
+                     if (!close(r++)) return false;
+                  CoarseCta &ct = T.ctas[cta0 + r];
+                  CoarseCell &ce = T.cells[(size_t)ct.cell0 + local[q]];
+                  ce.patch = ip;
+                  ce.lin = lin;
+                  if (ip == pe - 1) ce.last = (unsigned short)(ct.last = 1);
+                  const long long own1 = d.off1 + x[0] + 1 + step1[1] * (x[1] + 1) +
+                                         (dim == 3 ? step1[2] * (x[2] + 1) : 0);
+                  const int far = step[dim - 1];
+                  if (inner && x[0] > 0 && x[0] < n[0] - 1 && q - far >= first[r] &&
+                      q + far < first[r + 1]) {
+                     for (int a = 0; a < dim; ++a) {
+                        ce.nb[2 * a] = (unsigned short)local[q - step[a]];
+                        ce.nb[2 * a + 1] = (unsigned short)local[q + step[a]];
+                     }
+                     continue;
                   }
-                  int at = -1;
-                  if (m >= 0) {
-                     const int w = ord[(size_t)(m - base)];
-                     if (w < 0) return false;
-                     if (owner[w] == r) {
+                  for (int fc = 0; fc < 2 * dim; ++fc) {
+                     const int a = fc >> 1, s = fc & 1;
+                     int w = q + (s ? step[a] : -step[a]);
+                     long long m = own1 + (s ? step1[a] : -step1[a]);
+                     if (x[a] == (s ? n[a] - 1 : 0)) {
+                        const int t = a == 0 ? x[1] + n[1] * x[2]
+                                             : (a == 1 ? x[0] + n[0] * x[2] : x[0] + n[0] * x[1]);
+                        m = facemap[d.offo[a][s] + t];
+                        if (m == -1) {
+                           ghost[colour[q]].push_back({(unsigned)local[q], (unsigned)fc});
+                           continue;
+                        }
+                        if (m < 0) return false;  // neither a cell of the level nor a boundary
+                        // the cell of another patch that element m is
+                        int iq = pb;
+                        while (iq + 1 < pe && L.hp[iq + 1].off1 <= m) ++iq;
+                        const Box &bq = L.box[iq];
+                        const int mx = bq.hi[0] - bq.lo[0] + 1, my = bq.hi[1] - bq.lo[1] + 1;
+                        const long long e = m - L.hp[iq].off1, ez = e / ((long long)(mx + 2) * (my + 2));
+                        const long long er = e - ez * ((long long)(mx + 2) * (my + 2));
+                        w = pbase[iq - pb] + (int)(er % (mx + 2)) - 1 +
+                            mx * ((int)(er / (mx + 2)) - 1 + (dim == 3 ? my * ((int)ez - 1) : 0));
+                     }
+                     int at;
+                     if (w >= first[r] && w < first[r + 1]) {
                         at = local[w];
                      } else {
-                        if (pass == 0 && seen[w] != r) {
-                           // cells are visited CTA by CTA (owners ascend), so
-                           // seen and slot hold this CTA's copy
+                        if (seen[w] != r) {
                            seen[w] = r;
-                           slot[w] = nown + (int)halo[r].size();
+                           slot[w] = ct.ncol[0] + ct.ncol[1] + (int)halo[r].size();
                            halo[r].push_back(m);
-                           T.ctas[cta0 + r].nin[colour[w]] += 1;
-                           to[w].push_back((unsigned)r << 16 | (unsigned)slot[w]);
+                           ct.nin[colour[w]] += 1;
+                           to.push_back({w, (int)((long long)w * ncta / N),
+                                         (unsigned)r << 16 | ((unsigned)slot[w] & 0xffffu)});
                         }
-                        at = pass == 0 ? slot[w] : (int)ce.nb[fc];
+                        at = slot[w];
                      }
-                  } else if (m != -1) {
-                     return false;  // neither a cell of the level nor a physical boundary
-                  } else if (pass == 0) {
-                     ghost[2 * r + colour[q]].push_back((unsigned)fc << 16 | (unsigned)local[q]);
-                     at = 0;
-                  } else {
-                     at = nown + (int)halo[r].size() + gnext[2 * r + colour[q]]++ +
-                          (colour[q] ? (int)ghost[2 * r].size() : 0);
+                     if (at > 0xffff) return false;
+                     ce.nb[fc] = (unsigned short)at;
                   }
-                  if (at < 0 || at > 0xffff) return false;
-                  ce.nb[fc] = (unsigned short)at;
                }
             }
-         }
       }
-      for (int i = 0; i < (int)N; ++i) {
-         CoarseCell &ce = mine[owner[i]][local[i]];
-         ce.npush = (unsigned short)to[i].size();
-      }
-      std::vector<std::vector<int>> cell_of(ncta);
-      for (int r = 0; r < ncta; ++r) cell_of[r].resize(mine[r].size());
-      for (int i = 0; i < (int)N; ++i) cell_of[owner[i]][local[i]] = i;
-      for (int r = 0; r < ncta; ++r) {
+      for (; r < ncta; ++r)
+         if (!close(r)) return false;
+      std::stable_sort(to.begin(), to.end(), [&](const Push &x, const Push &y) {
+         return x.owner != y.owner ? x.owner < y.owner : local[x.cell] < local[y.cell];
+      });
+      size_t e = 0;
+      for (r = 0; r < ncta; ++r) {
          CoarseCta &ct = T.ctas[cta0 + r];
-         ct.cell0 = (int)T.cells.size();
          ct.halo0 = (int)T.halo.size();
+         T.halo.insert(T.halo.end(), halo[r].begin(), halo[r].end());
          ct.push0 = (int)T.push.size();
-         ct.nhalo = (int)halo[r].size();
-         ct.ghost0 = (int)T.ghost.size();
-         for (int k = 0; k < 2; ++k) {
-            ct.nghost[k] = (int)ghost[2 * r + k].size();
-            T.ghost.insert(T.ghost.end(), ghost[2 * r + k].begin(), ghost[2 * r + k].end());
-         }
-         for (size_t k = 0; k < mine[r].size(); ++k) {
-            mine[r][k].push0 = (int)T.push.size() - ct.push0;
-            const auto &t = to[cell_of[r][k]];
-            T.push.insert(T.push.end(), t.begin(), t.end());
+         for (int k = 0; k < ct.ncol[0] + ct.ncol[1]; ++k) {
+            CoarseCell &ce = T.cells[(size_t)ct.cell0 + k];
+            ce.push0 = (int)T.push.size() - ct.push0;
+            for (; e < to.size() && to[e].owner == r && local[to[e].cell] == k; ++e, ++ce.npush)
+               T.push.push_back(to[e].target);
          }
          ct.npush = (int)T.push.size() - ct.push0;
-         T.cells.insert(T.cells.end(), mine[r].begin(), mine[r].end());
-         T.halo.insert(T.halo.end(), halo[r].begin(), halo[r].end());
          const int ng = ct.nghost[0] + ct.nghost[1];
-         const long long nloc = (long long)mine[r].size() + ct.nhalo + ng;
+         const long long nloc = (long long)ct.ncol[0] + ct.ncol[1] + ct.nhalo + ng;
          const long long bytes = 8 * nloc + 8LL * ct.npush + 4LL * ng;
          if (nloc > 0xffff || bytes > kSolveSmemMax) return false;
          T.smem = std::max(T.smem, (int)((bytes + 15) / 16 * 16));
@@ -1746,6 +1777,9 @@ void build_coarse_solve(fac_ctx *c, const std::vector<long long> &facemap)
       L.coarse_sp = ch.sp;
       L.coarse_smem = T.smem;
       std::vector<unsigned char> all;
+      all.reserve(T.halo.size() * sizeof(long long) + T.ctas.size() * sizeof(CoarseCta) +
+                  T.cells.size() * sizeof(CoarseCell) +
+                  (T.push.size() + T.ghost.size()) * sizeof(unsigned) + 5 * 16);
       auto append = [&](int k, const void *src, size_t bytes) {
          L.coarse_at[k] = all.size();
          all.resize((all.size() + bytes + 15) / 16 * 16);
