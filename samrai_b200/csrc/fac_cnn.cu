@@ -1120,9 +1120,9 @@ int fac_cnn_create(fac_cnn **out, int device, int max_batch, unsigned long long 
        (rc = dalloc(n, &n->partial, kSumBlocks * sizeof(double))) ||
        (rc = dalloc(n, &n->done, sizeof(unsigned))))
       return fail(rc);
-   if (cudaHostAlloc((void **)&n->host, kBackBytes, cudaHostAllocDefault) != cudaSuccess) {
+   if (samrai_b200::pinned_alloc((void **)&n->host, kBackBytes) != cudaSuccess) {
       n->host = nullptr;
-      t_cnn_error = "cudaHostAlloc failed";
+      t_cnn_error = "no page-locked host memory";
       return fail(FAC_ERR_NOMEM);
    }
    for (size_t l = 0, at = 0; l < 4; at += kSizes[l++]) n->gw[l] = n->grads + at;

@@ -461,7 +461,7 @@ struct fac_ctx {
       void alloc(size_t n)
       {
          free();
-         CUDA_CHECK(cudaHostAlloc((void **)&dots, 3 * n * sizeof(double), cudaHostAllocDefault));
+         CUDA_CHECK(pinned_alloc((void **)&dots, 3 * n * sizeof(double)));
          coef[0] = dots + n;
          coef[1] = coef[0] + n;
       }
@@ -541,8 +541,7 @@ struct fac_ctx {
       void alloc(int np)
       {
          free();
-         CUDA_CHECK(cudaHostAlloc((void **)&acc, np * sizeof(double2) + sizeof(int),
-                                  cudaHostAllocDefault));
+         CUDA_CHECK(pinned_alloc((void **)&acc, np * sizeof(double2) + sizeof(int)));
          err = reinterpret_cast<int *>(acc + np);
          *err = 0;
       }

@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdint>
+#include <map>
 #include <mutex>
 #include <stdexcept>
 #include <unordered_map>
@@ -1992,6 +1993,22 @@ int resident_blocks(const void *fn)
 long long kernel_launch_count() { return g_launches.load(); }
 
 void add_kernel_launches(long long n) { g_launches += n; }
+
+cudaError_t pinned_alloc(void **p, size_t bytes)
+{
+   static std::mutex mutex;
+   static std::map<int, void *> kept;
+   int device = 0;
+   if (cudaGetDevice(&device) == cudaSuccess) {
+      std::lock_guard<std::mutex> lock(mutex);
+      void *&k = kept[device];
+      if (!k && cudaHostAlloc(&k, 64, cudaHostAllocDefault) != cudaSuccess) {
+         k = nullptr;
+         (void)cudaGetLastError();
+      }
+   }
+   return cudaHostAlloc(p, bytes, cudaHostAllocDefault);
+}
 
 namespace {
 

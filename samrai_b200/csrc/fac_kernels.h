@@ -13,6 +13,13 @@ long long kernel_launch_count();
 // graph (removed at capture, added per replay).
 void add_kernel_launches(long long n);
 
+// Page-locked host memory the GPU writes, freed with cudaFreeHost.  The driver
+// locks a block with the first such allocation and unlocks it with the last,
+// which takes 1 to 3.6 ms; inside a locked block one takes 4 us.  64 bytes per
+// device therefore stay allocated until the process ends, so that programs
+// which make one context or network after another pay for the block once.
+cudaError_t pinned_alloc(void **p, size_t bytes);
+
 // Staged colour pass (fac_stage.cu): units {patch, first copy, copies,
 // header} of the compacted list (active problems only) with their copy
 // lists and headers; stage_bytes is the largest StagePlan::bytes of the
