@@ -82,7 +82,7 @@ __device__ __forceinline__ void mma_bf16(float *d, const uint32_t *a, uint32_t b
 // (five tiles), the twenty others issue the copies of the next slab (cp.async)
 // and read, gate, round and store the half before, a tile per four warps.  One
 // CTA per SM.  What bounds it: the tensor cores read A from shared memory for
-// every MMA, 40 cycles for 128 rows with N = 16 and 70 with N = 48 (one or five
+// every MMA, 40 cycles for 128 rows with N = 16 and 64 with N = 48 (one or five
 // issuing threads alike), hence three taps per MMA; then the readers.  For 256
 // samples (ncu): 80 us a 16 -> 16 convolution and 53 us layer 4, 102 us each
 // with one MMA of N = 16 per tap and staging, multiplying and storing in turn

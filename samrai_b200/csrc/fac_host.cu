@@ -1388,7 +1388,7 @@ void build_residual_fixups(fac_ctx *c, int ln)
          if (mark[q]) L.rfix.push_back({ip, (int)q});
    }
    // the uncovered cells first: a residual that is restricted from the finer
-   // level next (residual_open) takes no others
+   // level next (comp_residual's open) takes no others
    const auto open = std::stable_partition(L.rfix.begin(), L.rfix.end(), [&](const CellRef &r) {
       return !L.cov[L.hp[r.patch].off0 + r.lin];
    });
@@ -1897,7 +1897,6 @@ void build_chunks(fac_ctx *c, int ln)
    L.fill_bytes = 16.0 * gcells;
 }
 
-// Inter-level tables with the next finer level (restriction, flux coarsening).
 // The cells of a level that lie under the next finer one.
 void build_covered(fac_ctx *c, int ln)
 {
@@ -1928,6 +1927,7 @@ void build_covered(fac_ctx *c, int ln)
    L.covered = L.n0 > 0 && n == L.n0;
 }
 
+// Inter-level tables with the next finer level (restriction, flux coarsening).
 void build_coarsen_tables(fac_ctx *c, int ln)
 {
    LevelState &C = c->L[ln];
@@ -2948,17 +2948,19 @@ void fac_cycle_recursive(fac_ctx *c, int ln)
 }
 
 // The first level the composite problem lives on.  The levels before it (a
-// coarse extension's) are covered throughout: u, the operator and the residual
-// there are restrictions of the finer level's, which a solve needs at its end
-// only (finish_low_levels) -- their weights are 0, they lend no ghost values,
-// and the cycle sets their right-hand sides and errors itself.
+// coarse extension's, or the caller's own) are covered throughout: u, the
+// operator and the residual there are restrictions of the finer level's, which
+// a solve needs at its end only (finish_low_levels) -- their weights are 0, they
+// lend no ghost values, and the cycle sets their right-hand sides and errors
+// itself.  A covered level is always one of them: what covers it has no
+// coarse-fine boundary, so it covers the domain.
 int first_level(const fac_ctx *c)
 {
    return c->cnn && c->learned_level < c->low ? 0 : c->low;
 }
 
-// u and the residual on those levels, as every cycle's restrictions would have
-// left them.
+// u with its ghost cells and the residual on those levels, as every cycle's
+// restrictions and fills would have left them.
 void finish_low_levels(fac_ctx *c)
 {
    for (int ln = first_level(c) - 1; ln >= 0; --ln) {
