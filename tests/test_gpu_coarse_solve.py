@@ -56,7 +56,11 @@ def _run(probs, bc, fused, sweeps, tol, data):
     for i, (e, r) in enumerate(data):
         g.upload(E, i, 0, e)
         g.upload(R, i, 0, r)
+    n0 = fac.kernel_launches()
     n = g.smooth(E, R, 0, sweeps, tol)
+    # the sweeps in one launch, or two colour passes and more for each
+    launches = fac.kernel_launches() - n0
+    assert launches <= 4 if fused else launches > 2 * int(n.max())
     out = [g.download(E, i, 0) for i in range(len(probs))]
     g.close()
     return n, out
